@@ -61,6 +61,7 @@ __device__ __forceinline__ MarchParams request_params(const BatchParams& bp, con
     p.K = q.sample_split;
     p.tm = make_tilemap(q.N, q.width, q.tile_w, q.tile_h);
     p.quad = q.vol_quad;
+    p.wide = wide_volume(q.D, q.H, q.W);
     p.qg = make_quadgeom(q.D, q.H, q.W);
     return p;
 }
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(256, 4) batched_fwd_kernel(const BatchParams b
         if (item >= bp.total) break;
         const int r = find_request(bp.off, bp.n_req, item);
         const MarchParams p = request_params(bp, bp.req[r], r);
-        if (p.quad != nullptr)
+        if (p.quad != nullptr && !p.wide)
             fwd_body<VT, VT, MULTI, 0, kLayoutQuad>(p, item - __ldg(bp.off + r), 0);
         else
             fwd_body<VT, VT, MULTI, 0, kLayoutVolume>(p, item - __ldg(bp.off + r), 0);

@@ -166,15 +166,15 @@ __device__ __forceinline__ float fix_frac(long long v) {
     return __int_as_float(0x3f800000u | ((unsigned)v >> 9)) - 1.0f;
 }
 
-// Nearest integer, ties to even (the nearest-label rule), on the exact value.
-__device__ __forceinline__ int fix_round(long long v) {
-    const int f = fix_floor(v);
+// Offset (0 or 1) of the nearest integer from the floor, ties to even (the
+// nearest-label rule), on the exact value.
+__device__ __forceinline__ int fix_near_offset(long long v) {
     const unsigned lo = (unsigned)v;
-    return f + ((lo > 0x80000000u) || (lo == 0x80000000u && (f & 1)) ? 1 : 0);
+    return (lo > 0x80000000u) | ((lo == 0x80000000u) & (fix_floor(v) & 1));
 }
 
-__device__ __forceinline__ FixPos fix_add(const FixPos& a, const FixPos& b) {
-    return FixPos{a.x + b.x, a.y + b.y, a.z + b.z};
+__device__ __forceinline__ int fix_round(long long v) {
+    return fix_floor(v) + fix_near_offset(v);
 }
 
 // Float-float helpers (value = hi + lo) for the per-ray set-up, written with
@@ -229,6 +229,7 @@ struct Cell {
     float v000, v001, v010, v011, v100, v101, v110, v111;  // v[z][y][x] offsets
     float fx, fy, fz;
     int ix, iy, iz;
+    int qi;   // quad layouts: element index of the cell in plane z0
     int cls;  // labelled quad layout only: class of the nearest corner (255 = dropped)
 };
 
@@ -307,7 +308,11 @@ __device__ __forceinline__ float cell_value(const Cell& c) {
 // Analytic derivative of the trilinear interpolant with respect to the
 // voxel-space position (the partial derivatives of the formula above).
 // Written with explicit fmaf so every kernel instantiation rounds the same
-// way (the compiler would otherwise be free to contract differently).
+// way (the compiler would otherwise be free to contract differently). A form
+// that shares the cross differences between the components takes 20
+// operations for 33 and was 1 to 5 % faster, but its rounding moved the
+// ill-conditioned rotation gradients of small one-pose steps by up to 1e-4,
+// so the rounding of this form stays.
 __device__ __forceinline__ void cell_grad(const Cell& c, float& gx, float& gy, float& gz) {
     const float wx0 = 1.f - c.fx, wy0 = 1.f - c.fy, wz0 = 1.f - c.fz;
     const float x00 = fmaf(c.v011 - c.v010, c.fy, __fmul_rn(c.v001 - c.v000, wy0));
@@ -321,82 +326,14 @@ __device__ __forceinline__ void cell_grad(const Cell& c, float& gx, float& gy, f
     gz = fmaf(z11, c.fy, __fmul_rn(z00, wy0));
 }
 
-// ---------------------------------------------- float positions (forward)
-// The forward evaluates sample positions in float32, as p0 + t * d with one
-// rounding (its images are within 1e-6 of the float64 oracle at 512^3); the
-// adjoint, whose gradients jump at cell faces, uses the fixed-point versions
-// below. Positions are clamped to [-2, dim + 1] first: beyond that every
-// corner is outside the volume either way, and the clamp keeps the float ->
-// int conversion in range for any input.
+// Two vector loads of the corners of quad element qi, planes z0 and z0 + 1.
 template <typename VT>
-__device__ __forceinline__ void load_cell(const VT* __restrict__ vol, int D, int H, int W, float x, float y,
-                                          float z, Cell& c) {
-    // Positions are clamped to [-2, dim + 1] first: beyond that every corner
-    // is outside the volume either way, and the clamp keeps the float -> int
-    // conversion in range for any input.
-    x = fminf(fmaxf(x, -2.0f), (float)W + 1.0f);
-    y = fminf(fmaxf(y, -2.0f), (float)H + 1.0f);
-    z = fminf(fmaxf(z, -2.0f), (float)D + 1.0f);
-    const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
-    c.fx = x - xf;
-    c.fy = y - yf;
-    c.fz = z - zf;
-    const int ix = (int)xf, iy = (int)yf, iz = (int)zf;
-    c.ix = ix;
-    c.iy = iy;
-    c.iz = iz;
-    const int HW = H * W;
-    const int base = (iz * H + iy) * W + ix;
-    if ((unsigned)ix < (unsigned)(W - 1) && (unsigned)iy < (unsigned)(H - 1) && (unsigned)iz < (unsigned)(D - 1)) {
-        c.v000 = ld_vox(vol, base);
-        c.v001 = ld_vox(vol, base + 1);
-        c.v010 = ld_vox(vol, base + W);
-        c.v011 = ld_vox(vol, base + W + 1);
-        c.v100 = ld_vox(vol, base + HW);
-        c.v101 = ld_vox(vol, base + HW + 1);
-        c.v110 = ld_vox(vol, base + HW + W);
-        c.v111 = ld_vox(vol, base + HW + W + 1);
-    } else {
-        const bool x0 = (unsigned)ix < (unsigned)W, x1 = (unsigned)(ix + 1) < (unsigned)W;
-        const bool y0 = (unsigned)iy < (unsigned)H, y1 = (unsigned)(iy + 1) < (unsigned)H;
-        const bool z0 = (unsigned)iz < (unsigned)D, z1 = (unsigned)(iz + 1) < (unsigned)D;
-        c.v000 = (z0 && y0 && x0) ? ld_vox(vol, base) : 0.f;
-        c.v001 = (z0 && y0 && x1) ? ld_vox(vol, base + 1) : 0.f;
-        c.v010 = (z0 && y1 && x0) ? ld_vox(vol, base + W) : 0.f;
-        c.v011 = (z0 && y1 && x1) ? ld_vox(vol, base + W + 1) : 0.f;
-        c.v100 = (z1 && y0 && x0) ? ld_vox(vol, base + HW) : 0.f;
-        c.v101 = (z1 && y0 && x1) ? ld_vox(vol, base + HW + 1) : 0.f;
-        c.v110 = (z1 && y1 && x0) ? ld_vox(vol, base + HW + W) : 0.f;
-        c.v111 = (z1 && y1 && x1) ? ld_vox(vol, base + HW + W + 1) : 0.f;
-    }
-}
-
-// Quad index of the cell whose lower corner is the floor of (x, y, z),
-// clamped into the padded extent, plus the fractional offsets and the cell's
-// (clamped) corner indices for the gradient scatter.
-__device__ __forceinline__ int quad_cell(const QuadGeom& g, int D, int H, int W, float x, float y, float z,
-                                         Cell& c) {
-    x = fminf(fmaxf(x, -2.0f), (float)W + 1.0f);
-    y = fminf(fmaxf(y, -2.0f), (float)H + 1.0f);
-    z = fminf(fmaxf(z, -2.0f), (float)D + 1.0f);
-    const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
-    c.fx = x - xf;
-    c.fy = y - yf;
-    c.fz = z - zf;
-    c.ix = min((int)xf, W);
-    c.iy = min((int)yf, H);
-    c.iz = min((int)zf, D);
-    return ((c.iz + 2) * g.qy + (c.iy + 2)) * g.qx + (c.ix + 2);
-}
-
-template <typename VT>
-__device__ __forceinline__ void load_cell_quad(const void* __restrict__ quad, const QuadGeom& g, int D, int H,
-                                               int W, float x, float y, float z, Cell& c) {
-    const int qi = quad_cell(g, D, H, W, x, y, z, c);
+__device__ __forceinline__ void load_quads(const void* __restrict__ quad, int plane, int qi, Cell& c) {
     using Q = typename QuadOf<VT>::T;
-    const Q* __restrict__ qp = reinterpret_cast<const Q*>(quad);
-    const Q q0 = __ldg(qp + qi);
-    const Q q1 = __ldg(qp + qi + g.plane);
+    const Q* __restrict__ q0p = reinterpret_cast<const Q*>(quad);
+    const Q* __restrict__ q1p = q0p + plane;
+    const Q q0 = __ldg(q0p + (unsigned)qi);
+    const Q q1 = __ldg(q1p + (unsigned)qi);
     if constexpr (std::is_same<VT, float>::value) {
         unpack_quad(q0, c.v000, c.v001, c.v010, c.v011);
         unpack_quad(q1, c.v100, c.v101, c.v110, c.v111);
@@ -409,14 +346,27 @@ __device__ __forceinline__ void load_cell_quad(const void* __restrict__ quad, co
     }
 }
 
-// Labelled quad at a float position (see load_cell_quad_labeled_fix).
+// Offset (0 or 1) of the nearest voxel from the cell's lower corner i: rint
+// with ties to even, read from the fraction (1 past one half, or at one half
+// on an odd corner).
+__device__ __forceinline__ int near_offset(float f, int i) {
+    return (f > 0.5f) | ((f == 0.5f) & (i & 1));
+}
+
+// Labelled quad layout (16-bit volumes): a 16-byte element holds the four
+// corner values of the plain 16-bit quad in .x/.y and the four corners'
+// classes (uint8, in the same corner order; 255 = dropped, 0 outside the
+// volume) in .z; .w is zero. The two loads of a sample then also carry the
+// classes of its eight corners, and the nearest one is picked from the
+// offsets ox, oy, oz of the nearest voxel (near_offset): byte ox + 2 oy of
+// plane oz's class word, one byte permute over both.
 template <typename VT>
-__device__ __forceinline__ void load_cell_quad_labeled(const void* __restrict__ quad, const QuadGeom& g, int D, int H,
-                                                       int W, float x, float y, float z, Cell& c) {
-    const int qi = quad_cell(g, D, H, W, x, y, z, c);
-    const uint4* __restrict__ qp = reinterpret_cast<const uint4*>(quad);
-    const uint4 q0 = __ldg(qp + qi);
-    const uint4 q1 = __ldg(qp + qi + g.plane);
+__device__ __forceinline__ void load_quads_labeled(const void* __restrict__ quad, int plane, int qi, int ox, int oy,
+                                                   int oz, Cell& c) {
+    const uint4* __restrict__ q0p = reinterpret_cast<const uint4*>(quad);
+    const uint4* __restrict__ q1p = q0p + plane;
+    const uint4 q0 = __ldg(q0p + (unsigned)qi);
+    const uint4 q1 = __ldg(q1p + (unsigned)qi);
     if constexpr (std::is_same<VT, __nv_bfloat16>::value) {
         unpack_quad_bf16(make_uint2(q0.x, q0.y), c.v000, c.v001, c.v010, c.v011);
         unpack_quad_bf16(make_uint2(q1.x, q1.y), c.v100, c.v101, c.v110, c.v111);
@@ -424,48 +374,57 @@ __device__ __forceinline__ void load_cell_quad_labeled(const void* __restrict__ 
         unpack_quad_f16(make_uint2(q0.x, q0.y), c.v000, c.v001, c.v010, c.v011);
         unpack_quad_f16(make_uint2(q1.x, q1.y), c.v100, c.v101, c.v110, c.v111);
     }
-    // Nearest corner, ties to even: rint of the clamped coordinate minus the
-    // cell's corner, read from the fraction quad_cell already formed (1 past
-    // one half, or at one half on an odd corner). Where the clamp moved the
-    // cell every corner lies outside the volume and carries class 0, so the
-    // choice there cannot change the class.
-    const int ox = (c.fx > 0.5f) | ((c.fx == 0.5f) & (c.ix & 1));
-    const int oy = (c.fy > 0.5f) | ((c.fy == 0.5f) & (c.iy & 1));
-    const int oz = (c.fz > 0.5f) | ((c.fz == 0.5f) & (c.iz & 1));
-    // byte ox + 2 oy of plane oz's class word: one byte permute over both
     c.cls = (int)(__byte_perm(q0.z, q1.z, (unsigned)(ox + 2 * oy + 4 * oz)) & 0xffu);
 }
 
-// Nearest-voxel label at (x, y, z); ties round to even like grid_sample's
-// nearest mode. Out-of-volume positions read label 0 (zero padding).
-__device__ __forceinline__ int nearest_label(const void* __restrict__ lab, int lab_dtype, int D, int H, int W,
-                                             float x, float y, float z) {
-    x = fminf(fmaxf(x, -2.0f), (float)W + 1.0f);
-    y = fminf(fmaxf(y, -2.0f), (float)H + 1.0f);
-    z = fminf(fmaxf(z, -2.0f), (float)D + 1.0f);
-    const int rx = (int)rintf(x), ry = (int)rintf(y), rz = (int)rintf(z);
-    if ((unsigned)rx < (unsigned)W && (unsigned)ry < (unsigned)H && (unsigned)rz < (unsigned)D)
-        return ld_label(lab, lab_dtype, (rz * H + ry) * W + rx);
-    return 0;
+// ------------------------------------- float positions inside the volume box
+// The march's loops run over samples whose cell has a corner in the volume
+// (lower corner in [-1, dim - 1] on every axis): the positions of a ray are
+// monotonic in the sample index, in float as in fixed point, so when the
+// first and last sample of a range are inside, all are, and the loop needs no
+// clamp per sample. Dropped samples have eight corners outside the volume.
+__device__ __forceinline__ bool pos_inside(float x, float y, float z, int D, int H, int W) {
+    return x >= -1.f && x < (float)W && y >= -1.f && y < (float)H && z >= -1.f && z < (float)D;
 }
 
-// Cell of a fixed-point position: the integer parts clamped into [-2, dim]
-// (a cell there has every corner outside the volume, so the clamp changes no
-// value or gradient, and it keeps quad indices inside the padded extent) and
-// the fractions of the unclamped position.
-__device__ __forceinline__ void fix_cell(const FixPos& P, int D, int H, int W, Cell& c) {
-    c.ix = min(max(fix_floor(P.x), -2), W);
-    c.iy = min(max(fix_floor(P.y), -2), H);
-    c.iz = min(max(fix_floor(P.z), -2), D);
-    c.fx = fix_frac(P.x);
-    c.fy = fix_frac(P.y);
-    c.fz = fix_frac(P.z);
+// floor(x) and x - floor(x) for |x| < 2^22 on the full-rate adder: adding
+// 1.5 * 2^23 rounding down leaves floor(x) in the low mantissa bits (ulp 1
+// there), where the conversion instructions (floor, float -> int) run at a
+// fraction of its rate. `bits` is floor(x) + 0x4b400000.
+constexpr float kFloorMagic = 12582912.0f;
+constexpr unsigned kFloorBits = 0x4b400000u;
+__device__ __forceinline__ unsigned floor_frac(float x, float& f) {
+    const float a = __fadd_rd(x, kFloorMagic);
+    f = x - (a - kFloorMagic);
+    return __float_as_uint(a);
 }
 
+// Lower corner, fractions and quad index of an inside position. The index is
+// formed from the biased floors; their bias leaves through `bias`
+// (quad_bias), all modulo 2^32.
+__device__ __forceinline__ unsigned quad_bias(const QuadGeom& g) {
+    const unsigned qx = (unsigned)g.qx, qy = (unsigned)g.qy;
+    return ((2u - kFloorBits) * qy + (2u - kFloorBits)) * qx + (2u - kFloorBits);
+}
+
+__device__ __forceinline__ void inside_cell(float x, float y, float z, Cell& c) {
+    c.ix = (int)(floor_frac(x, c.fx) - kFloorBits);
+    c.iy = (int)(floor_frac(y, c.fy) - kFloorBits);
+    c.iz = (int)(floor_frac(z, c.fz) - kFloorBits);
+}
+
+__device__ __forceinline__ void inside_quad(const QuadGeom& g, unsigned bias, float x, float y, float z, Cell& c) {
+    const unsigned bx = floor_frac(x, c.fx), by = floor_frac(y, c.fy), bz = floor_frac(z, c.fz);
+    c.qi = (int)((bz * (unsigned)g.qy + by) * (unsigned)g.qx + bx + bias);
+    c.ix = (int)(bx - kFloorBits);
+    c.iy = (int)(by - kFloorBits);
+    c.iz = (int)(bz - kFloorBits);
+}
+
+// The eight corners of cell (c.ix, c.iy, c.iz) from the plain volume, bounds
+// checked per corner where the cell crosses the border.
 template <typename VT>
-__device__ __forceinline__ void load_cell_fix(const VT* __restrict__ vol, int D, int H, int W, const FixPos& P,
-                                              Cell& c) {
-    fix_cell(P, D, H, W, c);
+__device__ __forceinline__ void load_corners(const VT* __restrict__ vol, int D, int H, int W, Cell& c) {
     const int ix = c.ix, iy = c.iy, iz = c.iz;
     const int HW = H * W;
     const int base = (iz * H + iy) * W + ix;
@@ -493,59 +452,51 @@ __device__ __forceinline__ void load_cell_fix(const VT* __restrict__ vol, int D,
     }
 }
 
-__device__ __forceinline__ int quad_index(const QuadGeom& g, const Cell& c) {
-    return ((c.iz + 2) * g.qy + (c.iy + 2)) * g.qx + (c.ix + 2);
+// The cell of any float position (clamped to [-2, dim + 1] first: beyond that
+// every corner is outside the volume either way, and the clamp keeps the
+// float -> int conversion in range for any input).
+template <typename VT>
+__device__ __forceinline__ void load_cell(const VT* __restrict__ vol, int D, int H, int W, float x, float y,
+                                          float z, Cell& c) {
+    x = fminf(fmaxf(x, -2.0f), (float)W + 1.0f);
+    y = fminf(fmaxf(y, -2.0f), (float)H + 1.0f);
+    z = fminf(fmaxf(z, -2.0f), (float)D + 1.0f);
+    const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
+    c.fx = x - xf;
+    c.fy = y - yf;
+    c.fz = z - zf;
+    c.ix = (int)xf;
+    c.iy = (int)yf;
+    c.iz = (int)zf;
+    load_corners(vol, D, H, W, c);
 }
 
-template <typename VT>
-__device__ __forceinline__ void load_cell_quad_fix(const void* __restrict__ quad, const QuadGeom& g, int D, int H,
-                                                   int W, const FixPos& P, Cell& c) {
-    fix_cell(P, D, H, W, c);
-    const int qi = quad_index(g, c);
-    using Q = typename QuadOf<VT>::T;
-    const Q* __restrict__ qp = reinterpret_cast<const Q*>(quad);
-    const Q q0 = __ldg(qp + qi);
-    const Q q1 = __ldg(qp + qi + g.plane);
-    if constexpr (std::is_same<VT, float>::value) {
-        unpack_quad(q0, c.v000, c.v001, c.v010, c.v011);
-        unpack_quad(q1, c.v100, c.v101, c.v110, c.v111);
-    } else if constexpr (std::is_same<VT, __nv_bfloat16>::value) {
-        unpack_quad_bf16(q0, c.v000, c.v001, c.v010, c.v011);
-        unpack_quad_bf16(q1, c.v100, c.v101, c.v110, c.v111);
-    } else {
-        unpack_quad_f16(q0, c.v000, c.v001, c.v010, c.v011);
-        unpack_quad_f16(q1, c.v100, c.v101, c.v110, c.v111);
-    }
+// Nearest-voxel label of an inside position whose cell is c (ties to even,
+// near_offset); a nearest voxel outside the volume reads label 0 (zero
+// padding).
+__device__ __forceinline__ int nearest_label(const void* __restrict__ lab, int lab_dtype, int D, int H, int W,
+                                             const Cell& c) {
+    const int rx = c.ix + near_offset(c.fx, c.ix), ry = c.iy + near_offset(c.fy, c.iy),
+              rz = c.iz + near_offset(c.fz, c.iz);
+    if ((unsigned)rx < (unsigned)W && (unsigned)ry < (unsigned)H && (unsigned)rz < (unsigned)D)
+        return ld_label(lab, lab_dtype, (rz * H + ry) * W + rx);
+    return 0;
 }
 
-// Labelled quad layout (16-bit volumes): a 16-byte element holds the four
-// corner values of the plain 16-bit quad in .x/.y and the four corners'
-// classes (uint8, in the same corner order; 255 = dropped, 0 outside the
-// volume) in .z; .w is zero. The two loads of a sample then also carry the
-// classes of its eight corners, and the nearest one is picked by rounding the
-// exact position (ties to even, the reference's nearest rule): its offsets
-// from the cell are 0 or 1 on each axis for any position the clamp left
-// alone; any other offset means the nearest voxel is outside the volume,
-// class 0.
-template <typename VT>
-__device__ __forceinline__ void load_cell_quad_labeled_fix(const void* __restrict__ quad, const QuadGeom& g, int D,
-                                                           int H, int W, const FixPos& P, Cell& c) {
-    fix_cell(P, D, H, W, c);
-    const int qi = quad_index(g, c);
-    const uint4* __restrict__ qp = reinterpret_cast<const uint4*>(quad);
-    const uint4 q0 = __ldg(qp + qi);
-    const uint4 q1 = __ldg(qp + qi + g.plane);
-    if constexpr (std::is_same<VT, __nv_bfloat16>::value) {
-        unpack_quad_bf16(make_uint2(q0.x, q0.y), c.v000, c.v001, c.v010, c.v011);
-        unpack_quad_bf16(make_uint2(q1.x, q1.y), c.v100, c.v101, c.v110, c.v111);
-    } else {
-        unpack_quad_f16(make_uint2(q0.x, q0.y), c.v000, c.v001, c.v010, c.v011);
-        unpack_quad_f16(make_uint2(q1.x, q1.y), c.v100, c.v101, c.v110, c.v111);
-    }
-    const int ox = fix_round(P.x) - c.ix, oy = fix_round(P.y) - c.iy, oz = fix_round(P.z) - c.iz;
-    const bool inside = (unsigned)ox <= 1u && (unsigned)oy <= 1u && (unsigned)oz <= 1u;
-    const unsigned labels = oz ? q1.z : q0.z;
-    c.cls = inside ? (int)((labels >> (8 * (ox + 2 * oy))) & 0xffu) : 0;
+// Fixed-point positions: inside test and cell of an inside position.
+__device__ __forceinline__ bool fix_inside(const FixPos& P, int D, int H, int W) {
+    return (unsigned)(fix_floor(P.x) + 1) <= (unsigned)W && (unsigned)(fix_floor(P.y) + 1) <= (unsigned)H &&
+           (unsigned)(fix_floor(P.z) + 1) <= (unsigned)D;
+}
+
+__device__ __forceinline__ void fix_cell(const FixPos& P, const QuadGeom& g, Cell& c) {
+    c.ix = fix_floor(P.x);
+    c.iy = fix_floor(P.y);
+    c.iz = fix_floor(P.z);
+    c.fx = fix_frac(P.x);
+    c.fy = fix_frac(P.y);
+    c.fz = fix_frac(P.z);
+    c.qi = ((c.iz + 2) * g.qy + (c.iy + 2)) * g.qx + (c.ix + 2);
 }
 
 // Nearest-voxel label at a fixed-point position (ties to even); positions

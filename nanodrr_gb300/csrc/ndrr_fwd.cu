@@ -44,7 +44,7 @@ cudaError_t launch_fwd(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaS
     const size_t smem = fwd_smem_bytes(a, ls);
     const bool multi = a.n_classes > 1;
     const int skip = a.skip_mode;
-    if (a.vol_quad != nullptr) {
+    if (a.vol_quad != nullptr && !p.wide) {
         if (a.out_dtype != a.vol_dtype) return cudaErrorNotSupported;
         return launch_fwd_quad(p, a.vol_dtype, multi, skip, a.quad_labels != 0, grid, block, smem, st);
     }

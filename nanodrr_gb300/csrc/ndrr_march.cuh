@@ -75,10 +75,18 @@ struct MarchParams {
     const void* quad;
     float* gquad;
     QuadGeom qg;
+    bool wide;  // a dimension of 2^22 voxels or more (float floors need the conversion)
     // launch shape
     TileMap tm;
     int tw, th, K;
 };
+
+// A volume whose float voxel positions the forward's fast floor does not cover
+// (floor_frac): its forward takes the volume layout's converting loop.
+__host__ __device__ __forceinline__ bool wide_volume(int D, int H, int W) {
+    constexpr int kWide = 1 << 22;
+    return D >= kWide || H >= kWide || W >= kWide;
+}
 
 constexpr int kSkipSteps = 256;  // distance-field steps per query before giving up
 
@@ -120,9 +128,13 @@ __device__ __forceinline__ void fix_ray(const MarchParams& p, const float (&m)[1
     tr.fd = FixPos{fd[0], fd[1], fd[2]};
 }
 
-// Fixed-point position of sample s.
+// Fixed-point position of sample s >= 0 (as an unsigned product modulo 2^64:
+// two multiply-adds per axis, where the signed one takes a third for the sign).
 __device__ __forceinline__ FixPos fix_at(const ThreadRay& tr, int s) {
-    return FixPos{tr.f0.x + (long long)s * tr.fd.x, tr.f0.y + (long long)s * tr.fd.y, tr.f0.z + (long long)s * tr.fd.z};
+    const unsigned long long u = (unsigned)s;
+    return FixPos{(long long)((unsigned long long)tr.f0.x + u * (unsigned long long)tr.fd.x),
+                  (long long)((unsigned long long)tr.f0.y + u * (unsigned long long)tr.fd.y),
+                  (long long)((unsigned long long)tr.f0.z + u * (unsigned long long)tr.fd.z)};
 }
 
 // Box-culled ray set-up (every thread of a ray computes the same window).
@@ -247,40 +259,60 @@ constexpr int kLayoutVolume = 0;   // the caller's [D, H, W] array, eight gather
 constexpr int kLayoutQuad = 1;     // quad layout, two vector loads
 constexpr int kLayoutQuadLab = 2;  // labelled quad layout (16-bit volumes): classes ride in the same loads
 
-// The eight corners of the sample's cell from the plain volume (bounds
-// checked per corner) or from the quad layouts (two vector loads), at a
-// float position (the forward) or a fixed-point one (the adjoint).
+// The cell of a sample whose float position lies inside (pos_inside): eight
+// corners from the plain volume or two vector loads of a quad layout.
 template <typename VT, int QUAD>
-__device__ __forceinline__ void fetch_cell(const MarchParams& p, float x, float y, float z, Cell& c) {
-    if constexpr (QUAD == kLayoutQuadLab) {
-        load_cell_quad_labeled<VT>(p.quad, p.qg, p.D, p.H, p.W, x, y, z, c);
-    } else if constexpr (QUAD == kLayoutQuad) {
-        load_cell_quad<VT>(p.quad, p.qg, p.D, p.H, p.W, x, y, z, c);
+__device__ __forceinline__ void fetch_cell(const MarchParams& p, unsigned bias, float x, float y, float z, Cell& c) {
+    if constexpr (QUAD == kLayoutVolume) {
+        inside_cell(x, y, z, c);
+        load_corners(reinterpret_cast<const VT*>(p.vol), p.D, p.H, p.W, c);
     } else {
-        load_cell(reinterpret_cast<const VT*>(p.vol), p.D, p.H, p.W, x, y, z, c);
+        inside_quad(p.qg, bias, x, y, z, c);
+        if constexpr (QUAD == kLayoutQuadLab) {
+            load_quads_labeled<VT>(p.quad, p.qg.plane, c.qi, near_offset(c.fx, c.ix), near_offset(c.fy, c.iy),
+                                   near_offset(c.fz, c.iz), c);
+        } else {
+            load_quads<VT>(p.quad, p.qg.plane, c.qi, c);
+        }
     }
 }
 
 // The cell of a sample known to have eight zero corners: its position and
 // weights, no loads.
 __device__ __forceinline__ void zero_cell(const MarchParams& p, const FixPos& P, Cell& c) {
-    fix_cell(P, p.D, p.H, p.W, c);
+    fix_cell(P, p.qg, c);
     c.v000 = c.v001 = c.v010 = c.v011 = c.v100 = c.v101 = c.v110 = c.v111 = 0.f;
     c.cls = 0;
 }
 
+// The same at an inside fixed-point position (the adjoint).
 template <typename VT, int QUAD>
 __device__ __forceinline__ void fetch_cell(const MarchParams& p, const FixPos& P, Cell& c) {
+    fix_cell(P, p.qg, c);
     if constexpr (QUAD == kLayoutQuadLab) {
-        load_cell_quad_labeled_fix<VT>(p.quad, p.qg, p.D, p.H, p.W, P, c);
+        load_quads_labeled<VT>(p.quad, p.qg.plane, c.qi, fix_near_offset(P.x), fix_near_offset(P.y),
+                               fix_near_offset(P.z), c);
     } else if constexpr (QUAD == kLayoutQuad) {
-        load_cell_quad_fix<VT>(p.quad, p.qg, p.D, p.H, p.W, P, c);
+        load_quads<VT>(p.quad, p.qg.plane, c.qi, c);
     } else {
-        load_cell_fix(reinterpret_cast<const VT*>(p.vol), p.D, p.H, p.W, P, c);
+        load_corners(reinterpret_cast<const VT*>(p.vol), p.D, p.H, p.W, c);
     }
 }
 
 // ===================================================================== forward
+// Samples per iteration of the forward loop, all cells loaded before any is
+// used (gathers in flight per thread), chosen together with the register
+// budgets (FwdRegs): the f32 quad with two samples and 48 registers marched
+// 512^3 x 32 x 256^2 x 800 in 2.05 ms (three samples 2.06 to 2.09, four 2.04
+// to 2.16, one 2.28), the labelled quad (bf16, 8 channels, 512 x 512 x 400)
+// with three and 64 registers in 2.18 ms (two 2.24, one 2.49). The volume
+// layout keeps one: its one-pose forward is DRAM-bound and lost resident CTAs
+// to a pair's registers (200^2 x 500 samples: 74 against 64 us).
+template <int QUAD>
+struct FwdUnroll {
+    static constexpr int value = QUAD == kLayoutQuad ? 2 : QUAD == kLayoutQuadLab ? 3 : 1;
+};
+
 // SKIP: 0 no skipping (or precomputed sample windows), 1 occupancy window.
 template <typename VT, typename OT, bool MULTI, int SKIP, int QUAD = kLayoutVolume>
 __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, const int b) {
@@ -317,8 +349,18 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
     if (MULTI) {
         for (int c = 0; c < p.C; ++c) cacc[c * NT] = 0.f;
     }
+    // Positions in float32, p0 + t * d with one rounding: the image is within
+    // 1e-6 of the float64 oracle at 512^3 (fixed-point positions, which the
+    // adjoint uses, measured 28 % slower here: 2.75 against 2.14 ms at
+    // 512^3 x 32 x 256^2).
+    auto at = [&](float sf, float& x, float& y, float& z) {
+        const float t = sf * p.inv_s;
+        x = fmaf(t, tr.ray.dx, tr.ray.p0x);
+        y = fmaf(t, tr.ray.dy, tr.ray.p0y);
+        z = fmaf(t, tr.ray.dz, tr.ray.p0z);
+    };
     // One sample's terms, in sample order.
-    auto take = [&](int s, float x, float y, float z, const Cell& cell) {
+    auto take = [&](int s, const Cell& cell) {
         const float val = cell_value(cell);
         acc += val;
         if (p.out_extent) {
@@ -334,7 +376,7 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
             if constexpr (QUAD == kLayoutQuadLab) {
                 cls = cell.cls;
             } else {
-                cls = nearest_label(p.lab, p.lab_dtype, p.D, p.H, p.W, x, y, z);
+                cls = nearest_label(p.lab, p.lab_dtype, p.D, p.H, p.W, cell);
             }
             if (cls != run_cls) {
                 if ((unsigned)run_cls < (unsigned)p.C) cacc[run_cls * NT] += run;
@@ -344,40 +386,53 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
             run += val;
         }
     };
-    // Quad layout: two samples per iteration, both cells loaded before either
-    // is used, so two gathers per thread are in flight (label gathers: 3.88
-    // against 4.28 ms at 512 x 512 x 400, 32 poses x 256^2, 8 channels; one
-    // channel 2.12 against 2.13). The labelled layout keeps one sample per
-    // iteration and trades registers for occupancy instead (2.88 ms, against
-    // 3.31 paired), and so does the volume layout, whose one-pose forward is
-    // DRAM-bound and lost resident CTAs to the pair's registers (64 against
-    // 56; 200^2 x 500 samples: 74 against 64 us per graph replay).
-    // Positions in float32, p0 + t * d with one rounding: the image is within
-    // 1e-6 of the float64 oracle at 512^3 and the loop stays near 56
-    // registers (fixed-point positions, which the adjoint uses, measured 28 %
-    // slower here: 2.75 against 2.14 ms at 512^3 x 32 x 256^2).
-    int s = tr.s0;
-    if constexpr (QUAD == kLayoutQuad) {
-        for (; s + 1 < tr.s1; s += 2) {
-            const float ta = (float)s * p.inv_s, tb = (float)(s + 1) * p.inv_s;
-            const float xa = fmaf(ta, tr.ray.dx, tr.ray.p0x), xb = fmaf(tb, tr.ray.dx, tr.ray.p0x);
-            const float ya = fmaf(ta, tr.ray.dy, tr.ray.p0y), yb = fmaf(tb, tr.ray.dy, tr.ray.p0y);
-            const float za = fmaf(ta, tr.ray.dz, tr.ray.p0z), zb = fmaf(tb, tr.ray.dz, tr.ray.p0z);
-            Cell ca, cb;
-            fetch_cell<VT, QUAD>(p, xa, ya, za, ca);
-            fetch_cell<VT, QUAD>(p, xb, yb, zb, cb);
-            take(s, xa, ya, za, ca);
-            take(s + 1, xb, yb, zb, cb);
+    // Trim the chunk to the samples whose cell has a corner in the volume;
+    // positions are monotonic in s, so the loops below need no clamp per
+    // sample. The window is a few samples wider than the box at its ends.
+    int s = tr.s0, s1 = tr.s1;
+    {
+        float x, y, z;
+        for (; s < s1; ++s) {
+            at((float)s, x, y, z);
+            if (pos_inside(x, y, z, p.D, p.H, p.W)) break;
+        }
+        for (; s < s1; --s1) {
+            at((float)(s1 - 1), x, y, z);
+            if (pos_inside(x, y, z, p.D, p.H, p.W)) break;
         }
     }
-    for (; s < tr.s1; ++s) {
-        const float t = (float)s * p.inv_s;
-        const float x = fmaf(t, tr.ray.dx, tr.ray.p0x);
-        const float y = fmaf(t, tr.ray.dy, tr.ray.p0y);
-        const float z = fmaf(t, tr.ray.dz, tr.ray.p0z);
+    const unsigned bias = quad_bias(p.qg);
+    if (QUAD == kLayoutVolume && p.wide) {
+        // a dimension of 2^22 voxels or more: floor by conversion
+        for (; s < s1; ++s) {
+            float x, y, z;
+            at((float)s, x, y, z);
+            Cell cell;
+            load_cell(reinterpret_cast<const VT*>(p.vol), p.D, p.H, p.W, x, y, z, cell);
+            take(s, cell);
+        }
+    }
+    constexpr int U = FwdUnroll<QUAD>::value;
+    if constexpr (U > 1) {
+        for (; s + (U - 1) < s1; s += U) {
+            const float sf = (float)s;
+            Cell c[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                float x, y, z;
+                at(sf + (float)j, x, y, z);
+                fetch_cell<VT, QUAD>(p, bias, x, y, z, c[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j) take(s + j, c[j]);
+        }
+    }
+    for (; s < s1; ++s) {
+        float x, y, z;
+        at((float)s, x, y, z);
         Cell cell;
-        fetch_cell<VT, QUAD>(p, x, y, z, cell);
-        take(s, x, y, z, cell);
+        fetch_cell<VT, QUAD>(p, bias, x, y, z, cell);
+        take(s, cell);
     }
     if (MULTI && (unsigned)run_cls < (unsigned)p.C) cacc[run_cls * NT] += run;
 
@@ -432,19 +487,17 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
 }
 
 // Register budget of the forward per instantiation, set for occupancy: the
-// loop is latency-bound, and more resident warps pay until spills cost more
-// (kernel alone, 512 x 512 x 400 f32 / bf16, 32 poses x 256^2, 800 samples):
-// f32 quad, one channel: 2.02 ms at 48 registers (10 CTAs of 128 per SM)
-// against 2.10 at 56 and 2.41 at 40; f32 quad, 8 channels with label
-// gathers: 3.77 at 40 against 3.81 at 48 and 3.93 at 64; labelled quad
-// (bf16, 8 channels): 2.88 at 40 against 2.99 at 48 and 3.18 at 52; the
-// volume layout: 3.59 at 64 against 3.83 at 48. Others keep 64 (two CTAs of
-// 512 threads per SM).
+// loop waits for its gathers, and more resident warps pay until spills cost
+// more (kernel alone, 512 x 512 x 400 / 512^3, 32 poses x 256^2, 800 samples):
+// f32 quad, one channel 2.05 ms at 48 registers (10 CTAs of 128 per SM), 2.11
+// at 56, 2.37 at 40; f32 quad, 8 channels with label gathers 3.59 at 56, 3.60
+// at 48, 4.08 at 40; 16-bit quad, one channel 1.37 at 40, 1.45 at 48, 1.55
+// at 64; the labelled quad 2.18 at 64, 2.22 at 72. The volume layout keeps 64
+// (3.45; 3.49 at 48).
 template <typename VT, bool MULTI, int QUAD>
 struct FwdRegs {
-    static constexpr int value = QUAD == kLayoutQuadLab ? 40
-                                 : (QUAD == kLayoutQuad && std::is_same<VT, float>::value) ? (MULTI ? 40 : 48)
-                                                                                            : 64;
+    static constexpr bool f32 = std::is_same<VT, float>::value;
+    static constexpr int value = QUAD != kLayoutQuad ? 64 : f32 ? (MULTI ? 56 : 48) : (MULTI ? 64 : 40);
 };
 
 template <typename VT, typename OT, bool MULTI, int SKIP, int QUAD>
@@ -461,17 +514,17 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // Per-thread adjoint accumulators. The pose partial of a ray is
 //   dL/dM_ij = sum_s g_s dv_s,i [q_s, 1]_j,  q_s = src + t_s e,
-// which this thread keeps as two 3-vectors, G = sum_s g_s dv_s and
-// Gt = sum_s g_s dv_s t_s (6 multiply-adds per sample instead of 12 plus the
-// position q_s), and expands once per ray: dL/dM_ij = G_i src_j + Gt_i e_j for
-// j < 3, dL/dM_i3 = G_i (pose_terms).
+// and its camera gradients are M^T sum_s (1 - t_s) g_s dv_s (source) and
+// M^T sum_s t_s g_s dv_s (target), so a thread keeps two 3-vectors, G =
+// sum_s g_s dv_s and Gt = sum_s g_s dv_s t_s (6 operations per sample), and
+// expands them once per ray. V = sum_s w_s v_s (camera gradients only; w the
+// upstream gradient) is the derivative in the ray's step.
 struct AdjAcc {
-    float G[3], Gt[3];
-    float gsx, gsy, gsz, gtx, gty, gtz, gst;
+    float G[3], Gt[3], V;
     __device__ __forceinline__ void zero() {
 #pragma unroll
         for (int j = 0; j < 3; ++j) G[j] = Gt[j] = 0.f;
-        gsx = gsy = gsz = gtx = gty = gtz = gst = 0.f;
+        V = 0.f;
     }
     __device__ __forceinline__ void pose_terms(float sx, float sy, float sz, float ex, float ey, float ez,
                                                float (&a)[12]) const {
@@ -489,9 +542,9 @@ struct AdjAcc {
 struct DirectScatter {
     float* __restrict__ gvol;
     int D, H, W;
-    __device__ __forceinline__ void operator()(int idx_unused, int ix, int iy, int iz, float g00, float g01,
-                                               float g10, float g11, float wx0, float wx1) const {
-        (void)idx_unused;
+    __device__ __forceinline__ void operator()(const Cell& c, float g00, float g01, float g10, float g11, float wx0,
+                                               float wx1) const {
+        const int ix = c.ix, iy = c.iy, iz = c.iz;
         const int HW = H * W;
         const int base = (iz * H + iy) * W + ix;
         if ((unsigned)ix < (unsigned)(W - 1) && (unsigned)iy < (unsigned)(H - 1) && (unsigned)iz < (unsigned)(D - 1)) {
@@ -526,8 +579,9 @@ struct BrickScatter {
     float* acc;
     int D, H, W;
     int x0, y0, z0, nx, ny;
-    __device__ __forceinline__ void operator()(int, int ix, int iy, int iz, float g00, float g01, float g10,
-                                               float g11, float wx0, float wx1) const {
+    __device__ __forceinline__ void operator()(const Cell& c, float g00, float g01, float g10, float g11, float wx0,
+                                               float wx1) const {
+        const int ix = c.ix, iy = c.iy, iz = c.iz;
         const int lx = ix - x0, ly = iy - y0, lz = iz - z0;
         const int nxy = nx * ny;
         const int base = (lz * ny + ly) * nx + lx;
@@ -553,11 +607,10 @@ struct BrickScatter {
 struct QuadScatter {
     float* __restrict__ gq;
     QuadGeom g;
-    __device__ __forceinline__ void operator()(int, int ix, int iy, int iz, float g00, float g01, float g10,
-                                               float g11, float wx0, float wx1) const {
-        const int qi = ((iz + 2) * g.qy + (iy + 2)) * g.qx + (ix + 2);
-        float* a = gq + (size_t)qi * 4;
-        float* b = a + (size_t)g.plane * 4;
+    __device__ __forceinline__ void operator()(const Cell& c, float g00, float g01, float g10, float g11, float wx0,
+                                               float wx1) const {
+        float* a = gq + (size_t)(unsigned)c.qi * 4;
+        float* b = gq + (size_t)g.plane * 4 + (size_t)(unsigned)c.qi * 4;
         // No "memory" clobber: nothing in the adjoint reads the gradient, so
         // the volume loads of later samples may be scheduled above these.
         asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a), "f"(g00 * wx0), "f"(g00 * wx1),
@@ -577,9 +630,9 @@ struct QuadScatter {
 struct QuadScatterWarp {
     float* __restrict__ gq;
     QuadGeom g;
-    __device__ __forceinline__ void operator()(int, int ix, int iy, int iz, float g00, float g01, float g10,
-                                               float g11, float wx0, float wx1) const {
-        const int qi = ((iz + 2) * g.qy + (iy + 2)) * g.qx + (ix + 2);
+    __device__ __forceinline__ void operator()(const Cell& c, float g00, float g01, float g10, float g11, float wx0,
+                                               float wx1) const {
+        const int qi = c.qi;
         const unsigned mask = __activemask();
         const int lane = threadIdx.x & 31;
         const unsigned peers = __match_any_sync(mask, qi);
@@ -624,87 +677,11 @@ __device__ __forceinline__ float sample_go(const MarchParams& p, int b, const Th
     return class_go(p, b, tr, nearest_label_fix(p.lab, p.lab_dtype, p.D, p.H, p.W, P));
 }
 
-// Adjoint terms of one sample whose cell is loaded.
+// Adjoint terms of one sample whose cell is loaded: w its upstream gradient,
+// g = w * step, t its ray parameter.
 template <bool GVOL, bool GCAM, typename Scatter>
-__device__ __forceinline__ void adjoint_accumulate(const float (&m)[12], const ThreadRay& tr, float t, float gg,
-                                                   const Cell& cell, AdjAcc& A, const Scatter& scatter);
-
-// Adjoint of samples [s0, s1) of one ray (reference _fused.py:230-298).
-// Samples go in pairs: both pairs' loads are issued before either's
-// reductions, so two gathers per thread are in flight. The accumulation
-// order is the sample order either way.
-template <typename VT, bool MULTI, bool GVOL, bool GCAM, typename Scatter, int QUAD = kLayoutVolume>
-__device__ __forceinline__ void adjoint_samples(const MarchParams& p, const float (&m)[12], const ThreadRay& tr,
-                                                int b, int s0, int s1, float go_ray, AdjAcc& A,
-                                                const Scatter& scatter) {
-    if (!MULTI && go_ray == 0.f) return;  // every term is proportional to go
-    // Each sample's position is formed from its index (f0 + s * step), not
-    // stepped from the previous one: stepping chains every load address to
-    // the last iteration's 64-bit add and measured 4.1 against 2.9 ms for the
-    // pose adjoint at 512^3 x 32 x 256^2; independent positions let the loads
-    // of later samples issue early, as with float positions.
-    int s = s0;
-    if constexpr (QUAD == kLayoutQuadLab) {
-        // the class of a sample arrives with its corners: fetch, then route
-        for (; s + 1 < s1; s += 2) {
-            const float ta = (float)s * p.inv_s, tb = (float)(s + 1) * p.inv_s;
-            const FixPos Pa = fix_at(tr, s), Pb = fix_at(tr, s + 1);
-            Cell ca, cb;
-            fetch_cell<VT, QUAD>(p, Pa, ca);
-            fetch_cell<VT, QUAD>(p, Pb, cb);
-            const float ga = MULTI ? class_go(p, b, tr, ca.cls) : go_ray;
-            const float gb = MULTI ? class_go(p, b, tr, cb.cls) : go_ray;
-            if (ga != 0.f) adjoint_accumulate<GVOL, GCAM>(m, tr, ta, ga, ca, A, scatter);
-            if (gb != 0.f) adjoint_accumulate<GVOL, GCAM>(m, tr, tb, gb, cb, A, scatter);
-        }
-        if (s < s1) {
-            const float t = (float)s * p.inv_s;
-            Cell cell;
-            fetch_cell<VT, QUAD>(p, fix_at(tr, s), cell);
-            const float gg = MULTI ? class_go(p, b, tr, cell.cls) : go_ray;
-            if (gg != 0.f) adjoint_accumulate<GVOL, GCAM>(m, tr, t, gg, cell, A, scatter);
-        }
-        return;
-    }
-    // Samples outside [glo, ghi) have eight zero corners (the window of an
-    // exact skip): no pose terms, so their cells are not loaded, while their
-    // volume-gradient terms (which need no corner values) are scattered.
-    for (; s + 1 < s1; s += 2) {
-        const float ta = (float)s * p.inv_s, tb = (float)(s + 1) * p.inv_s;
-        const FixPos Pa = fix_at(tr, s), Pb = fix_at(tr, s + 1);
-        const float ga = sample_go<MULTI>(p, b, tr, go_ray, Pa);
-        const float gb = sample_go<MULTI>(p, b, tr, go_ray, Pb);
-        Cell ca, cb;
-        if (MULTI || (s >= tr.glo && s < tr.ghi))
-            fetch_cell<VT, QUAD>(p, Pa, ca);
-        else
-            zero_cell(p, Pa, ca);
-        if (MULTI || (s + 1 >= tr.glo && s + 1 < tr.ghi))
-            fetch_cell<VT, QUAD>(p, Pb, cb);
-        else
-            zero_cell(p, Pb, cb);
-        if (ga != 0.f) adjoint_accumulate<GVOL, GCAM>(m, tr, ta, ga, ca, A, scatter);
-        if (gb != 0.f) adjoint_accumulate<GVOL, GCAM>(m, tr, tb, gb, cb, A, scatter);
-    }
-    if (s < s1) {
-        const float t = (float)s * p.inv_s;
-        const FixPos Pa = fix_at(tr, s);
-        const float gg = sample_go<MULTI>(p, b, tr, go_ray, Pa);
-        if (gg != 0.f) {
-            Cell cell;
-            if (MULTI || (s >= tr.glo && s < tr.ghi))
-                fetch_cell<VT, QUAD>(p, Pa, cell);
-            else
-                zero_cell(p, Pa, cell);
-            adjoint_accumulate<GVOL, GCAM>(m, tr, t, gg, cell, A, scatter);
-        }
-    }
-}
-
-template <bool GVOL, bool GCAM, typename Scatter>
-__device__ __forceinline__ void adjoint_accumulate(const float (&m)[12], const ThreadRay& tr, float t, float gg,
-                                                   const Cell& cell, AdjAcc& A, const Scatter& scatter) {
-    const float g = gg * tr.stepv;
+__device__ __forceinline__ void adjoint_accumulate(float t, float w, float g, const Cell& cell, AdjAcc& A,
+                                                   const Scatter& scatter) {
     float dvx, dvy, dvz;
     cell_grad(cell, dvx, dvy, dvz);
     const float gx = g * dvx, gy = g * dvy, gz = g * dvz;
@@ -714,24 +691,80 @@ __device__ __forceinline__ void adjoint_accumulate(const float (&m)[12], const T
     A.Gt[0] = fmaf(gx, t, A.Gt[0]);
     A.Gt[1] = fmaf(gy, t, A.Gt[1]);
     A.Gt[2] = fmaf(gz, t, A.Gt[2]);
-    if (GCAM) {
-        // Chain to camera space: gq = M[:, :3]^T gpos.
-        const float gqx = m[0] * gx + m[4] * gy + m[8] * gz;
-        const float gqy = m[1] * gx + m[5] * gy + m[9] * gz;
-        const float gqz = m[2] * gx + m[6] * gy + m[10] * gz;
-        const float omt = 1.f - t;
-        A.gsx = fmaf(omt, gqx, A.gsx);
-        A.gsy = fmaf(omt, gqy, A.gsy);
-        A.gsz = fmaf(omt, gqz, A.gsz);
-        A.gtx = fmaf(t, gqx, A.gtx);
-        A.gty = fmaf(t, gqy, A.gty);
-        A.gtz = fmaf(t, gqz, A.gtz);
-        A.gst = fmaf(gg, cell_value(cell), A.gst);
-    }
+    if (GCAM) A.V = fmaf(w, cell_value(cell), A.V);
     if (GVOL) {
         const float wy0 = 1.f - cell.fy, wz0 = 1.f - cell.fz;
-        scatter(0, cell.ix, cell.iy, cell.iz, g * wz0 * wy0, g * wz0 * cell.fy, g * cell.fz * wy0,
-                g * cell.fz * cell.fy, 1.f - cell.fx, cell.fx);
+        scatter(cell, g * wz0 * wy0, g * wz0 * cell.fy, g * cell.fz * wy0, g * cell.fz * cell.fy, 1.f - cell.fx,
+                cell.fx);
+    }
+}
+
+// Trims [s0, s1) of a ray to the samples whose cell has a corner in the
+// volume (fix_inside; the window is a few samples wider than the box at its
+// ends). Positions are linear in s, so with both ends inside every sample
+// between them is, and the loops need no clamp. That holds while s * step
+// does not wrap in 64 bits, which the last check decides from the step alone
+// (whole voxels per sample times samples, against the widest axis); a ray so
+// long that it wraps keeps its first inside sample.
+__device__ __forceinline__ void trim_inside(const MarchParams& p, const ThreadRay& tr, int& s0, int& s1) {
+    while (s0 < s1 && !fix_inside(fix_at(tr, s0), p.D, p.H, p.W)) ++s0;
+    while (s0 < s1 && !fix_inside(fix_at(tr, s1 - 1), p.D, p.H, p.W)) --s1;
+    const long long n1 = (long long)(s1 - s0) - 1, most = (long long)max(p.W, max(p.H, p.D)) + 2;
+    const long long vx = (tr.fd.x ^ (tr.fd.x >> 63)) >> 32, vy = (tr.fd.y ^ (tr.fd.y >> 63)) >> 32,
+                    vz = (tr.fd.z ^ (tr.fd.z >> 63)) >> 32;
+    if (n1 > 0 && max(vx, max(vy, vz)) * n1 > most) s1 = s0 + 1;
+}
+
+// Adjoint of samples [s0, s1) of one ray (reference _fused.py:230-298).
+// Samples go in pairs: both pairs' loads are issued before either's
+// reductions, so two gathers per thread are in flight. The accumulation
+// order is the sample order either way.
+template <typename VT, bool MULTI, bool GVOL, bool GCAM, typename Scatter, int QUAD = kLayoutVolume>
+__device__ __forceinline__ void adjoint_samples(const MarchParams& p, const ThreadRay& tr, int b, int s0, int s1,
+                                                float go_ray, AdjAcc& A, const Scatter& scatter) {
+    if (!MULTI && go_ray == 0.f) return;  // every term is proportional to go
+    trim_inside(p, tr, s0, s1);
+    // Each sample's position is formed from its index (f0 + s * step), not
+    // stepped from the previous one: stepping chains every load address to
+    // the last iteration's 64-bit add and measured 4.1 against 2.9 ms for the
+    // pose adjoint at 512^3 x 32 x 256^2; independent positions let the loads
+    // of later samples issue early, as with float positions.
+    //
+    // Samples outside [glo, ghi) have eight zero corners (the window of an
+    // exact skip): no pose terms, so their cells are not loaded, while their
+    // volume-gradient terms (which need no corner values) are scattered.
+    auto fetch = [&](int s, const FixPos& P, Cell& c) {
+        if (!GVOL || MULTI || (s >= tr.glo && s < tr.ghi))
+            fetch_cell<VT, QUAD>(p, P, c);
+        else
+            zero_cell(p, P, c);
+    };
+    // upstream gradient of a sample: the labelled layout's class arrives with
+    // its corners (fetch, then route)
+    auto route = [&](const FixPos& P, const Cell& c) {
+        if (QUAD == kLayoutQuadLab) return class_go(p, b, tr, c.cls);
+        return sample_go<MULTI>(p, b, tr, go_ray, P);
+    };
+    auto take = [&](float sf, float w, const Cell& c) {
+        if (MULTI && w == 0.f) return;
+        adjoint_accumulate<GVOL, GCAM>(sf * p.inv_s, w, w * tr.stepv, c, A, scatter);
+    };
+    int s = s0;
+    for (; s + 1 < s1; s += 2) {
+        const float sf = (float)s;
+        const FixPos Pa = fix_at(tr, s), Pb = fix_at(tr, s + 1);
+        Cell ca, cb;
+        fetch(s, Pa, ca);
+        fetch(s + 1, Pb, cb);
+        const float wa = route(Pa, ca), wb = route(Pb, cb);
+        take(sf, wa, ca);
+        take(sf + 1.f, wb, cb);
+    }
+    if (s < s1) {
+        const FixPos P = fix_at(tr, s);
+        Cell c;
+        fetch(s, P, c);
+        take((float)s, route(P, c), c);
     }
 }
 
@@ -739,9 +772,9 @@ __device__ __forceinline__ void adjoint_accumulate(const float (&m)[12], const T
 // pose partials into `partials[slot]`, and the per-ray camera
 // gradients (summing the K sample chunks of each ray in order).
 template <bool GCAM>
-__device__ __forceinline__ void adjoint_epilogue(const MarchParams& p, const size_t slot, const ThreadRay& tr,
-                                                 const AdjAcc& A,
-                                                 float* smem, int R, int NT, int r, int k) {
+__device__ __forceinline__ void adjoint_epilogue(const MarchParams& p, const float (&m)[12], const size_t slot,
+                                                 const ThreadRay& tr, const AdjAcc& A, float* smem, int R, int NT,
+                                                 int r, int k) {
     const int tid = threadIdx.x;
     const bool shared_src = GCAM && !p.src_per_ray;
     const int nwarps = NT >> 5;
@@ -749,6 +782,16 @@ __device__ __forceinline__ void adjoint_epilogue(const MarchParams& p, const siz
     float* wred = smem;  // [nwarps][kPartialStride]
     float a[12];
     A.pose_terms(tr.sx, tr.sy, tr.sz, tr.ex, tr.ey, tr.ez, a);
+    // camera space: M[:, :3]^T of the sums over (1 - t) and t
+    float gs[3], gt[3];
+    if (GCAM) {
+        const float h0 = A.G[0] - A.Gt[0], h1 = A.G[1] - A.Gt[1], h2 = A.G[2] - A.Gt[2];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            gs[j] = m[j] * h0 + m[4 + j] * h1 + m[8 + j] * h2;
+            gt[j] = m[j] * A.Gt[0] + m[4 + j] * A.Gt[1] + m[8 + j] * A.Gt[2];
+        }
+    }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < 12; ++j) {
@@ -756,7 +799,7 @@ __device__ __forceinline__ void adjoint_epilogue(const MarchParams& p, const siz
         if (lane == 0) wred[warp * kPartialStride + j] = v;
     }
     if (shared_src) {
-        const float v0 = warp_sum(A.gsx), v1 = warp_sum(A.gsy), v2 = warp_sum(A.gsz);
+        const float v0 = warp_sum(gs[0]), v1 = warp_sum(gs[1]), v2 = warp_sum(gs[2]);
         if (lane == 0) {
             wred[warp * kPartialStride + 12] = v0;
             wred[warp * kPartialStride + 13] = v1;
@@ -773,13 +816,13 @@ __device__ __forceinline__ void adjoint_epilogue(const MarchParams& p, const siz
     if (GCAM) {
         __syncthreads();
         float* cr = smem;  // [7][NT]
-        cr[0 * NT + tid] = A.gtx;
-        cr[1 * NT + tid] = A.gty;
-        cr[2 * NT + tid] = A.gtz;
-        cr[3 * NT + tid] = A.gst;
-        cr[4 * NT + tid] = A.gsx;
-        cr[5 * NT + tid] = A.gsy;
-        cr[6 * NT + tid] = A.gsz;
+        cr[0 * NT + tid] = gt[0];
+        cr[1 * NT + tid] = gt[1];
+        cr[2 * NT + tid] = gt[2];
+        cr[3 * NT + tid] = A.V;
+        cr[4 * NT + tid] = gs[0];
+        cr[5 * NT + tid] = gs[1];
+        cr[6 * NT + tid] = gs[2];
         __syncthreads();
         if (k == 0 && tr.n >= 0) {
             float v[7];
@@ -895,27 +938,25 @@ __device__ __forceinline__ void bwd_body(const MarchParams& p, const int tile, c
     A.zero();
     if constexpr (QUAD != kLayoutVolume && WARP_AGG) {
         const QuadScatterWarp sc{p.gquad, p.qg};
-        adjoint_samples<VT, MULTI, GVOL, GCAM, QuadScatterWarp, QUAD>(p, m, tr, b, tr.s0, tr.s1, go_ray, A, sc);
+        adjoint_samples<VT, MULTI, GVOL, GCAM, QuadScatterWarp, QUAD>(p, tr, b, tr.s0, tr.s1, go_ray, A, sc);
     } else if constexpr (QUAD != kLayoutVolume) {
         const QuadScatter sc{p.gquad, p.qg};
-        adjoint_samples<VT, MULTI, GVOL, GCAM, QuadScatter, QUAD>(p, m, tr, b, tr.s0, tr.s1, go_ray, A, sc);
+        adjoint_samples<VT, MULTI, GVOL, GCAM, QuadScatter, QUAD>(p, tr, b, tr.s0, tr.s1, go_ray, A, sc);
     } else {
         const DirectScatter sc{p.gvol, p.D, p.H, p.W};
-        adjoint_samples<VT, MULTI, GVOL, GCAM>(p, m, tr, b, tr.s0, tr.s1, go_ray, A, sc);
+        adjoint_samples<VT, MULTI, GVOL, GCAM>(p, tr, b, tr.s0, tr.s1, go_ray, A, sc);
     }
-    adjoint_epilogue<GCAM>(p, slot, tr, A, smem, R, NT, r, k);
+    adjoint_epilogue<GCAM>(p, m, slot, tr, A, smem, R, NT, r, k);
 }
 
 // Register budget of the adjoint: 128 (one CTA of 512 threads per SM), but
-// 56 for the one-channel pose-only adjoint of an f32 quad volume without an
-// in-kernel skip, where occupancy pays: 2.80 against 2.86 ms at 70
-// registers (512^3, 32 poses x 256^2, 800 samples, kernel alone; 64
-// measured 3.16).
+// 72 for the one-channel pose-only adjoint of an f32 quad volume without an
+// in-kernel skip, where occupancy pays: 0.70 ms, against 0.78 at 56 and 0.73
+// at 80 (512 x 512 x 400, 16 poses x 200^2, 500 samples, kernel alone).
 template <typename VT, bool MULTI, bool GVOL, bool GCAM, int SKIP, int QUAD>
 struct BwdRegs {
     static constexpr int value =
-        (!MULTI && !GVOL && !GCAM && SKIP == 0 && QUAD == kLayoutQuad && std::is_same<VT, float>::value) ? 56
-                                                                                                          : 128;
+        (!MULTI && !GVOL && !GCAM && SKIP == 0 && QUAD == kLayoutQuad && std::is_same<VT, float>::value) ? 72 : 128;
 };
 
 template <typename VT, bool MULTI, bool GVOL, bool GCAM, int SKIP, int QUAD>
@@ -1031,7 +1072,7 @@ __global__ void __launch_bounds__(256, 2) raymarch_bwd_brick_kernel(const MarchP
             for (int i = (n4 << 2) + tid; i < (int)nvox; i += NT) acc[i] = 0.f;
             __syncthreads();
             const BrickScatter sc{acc, p.D, p.H, p.W, lo3[0], lo3[1], lo3[2], nx, ny};
-            adjoint_samples<VT, MULTI, true, GCAM>(p, m, tr, b, a, e, go_ray, A, sc);
+            adjoint_samples<VT, MULTI, true, GCAM>(p, tr, b, a, e, go_ray, A, sc);
             __syncthreads();
             // Flush: each warp takes whole rows so lanes write consecutive x.
             const int warp = tid >> 5, lane = tid & 31;
@@ -1048,12 +1089,12 @@ __global__ void __launch_bounds__(256, 2) raymarch_bwd_brick_kernel(const MarchP
             if (nvox * 4 < cap) L = min(L * 2, 256);
         } else {
             const DirectScatter sc{p.gvol, p.D, p.H, p.W};
-            adjoint_samples<VT, MULTI, true, GCAM>(p, m, tr, b, a, e, go_ray, A, sc);
+            adjoint_samples<VT, MULTI, true, GCAM>(p, tr, b, a, e, go_ray, A, sc);
             if (nvox > cap) L = max(L >> 1, 2);
         }
         sb = se;
     }
-    adjoint_epilogue<GCAM>(p, blockIdx.x, tr, A, smem, R, NT, tid, 0);
+    adjoint_epilogue<GCAM>(p, m, blockIdx.x, tr, A, smem, R, NT, tid, 0);
 }
 
 // Per-pose sum of the per-tile partials in a fixed order. One CTA per pose.

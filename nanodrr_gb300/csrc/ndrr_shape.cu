@@ -49,6 +49,7 @@ MarchParams make_params(const ndrr_raymarch_args& a, const LaunchShape& ls) {
     p.quad = a.vol_quad;
     p.gquad = a.gvol_quad;
     p.qg = make_quadgeom(a.D, a.H, a.W);
+    p.wide = wide_volume(a.D, a.H, a.W);
     p.tw = ls.tw;
     p.th = ls.th;
     p.K = ls.K;

@@ -285,11 +285,13 @@ __device__ __forceinline__ void scatter_body(const MarchParams& p, const int til
     if (go == 0.f) return;  // every term is proportional to go
     const float g = go * tr.stepv;
     const QuadScatter sc{p.gquad, p.qg};
-    for (int s = tr.ray.lo; s < tr.ray.hi; ++s) {
+    int s0 = tr.ray.lo, s1 = tr.ray.hi;
+    trim_inside(p, tr, s0, s1);
+    for (int s = s0; s < s1; ++s) {
         Cell c;
-        fix_cell(fix_at(tr, s), p.D, p.H, p.W, c);
+        fix_cell(fix_at(tr, s), p.qg, c);
         const float wy0 = 1.f - c.fy, wz0 = 1.f - c.fz;
-        sc(0, c.ix, c.iy, c.iz, g * wz0 * wy0, g * wz0 * c.fy, g * c.fz * wy0, g * c.fz * c.fy, 1.f - c.fx, c.fx);
+        sc(c, g * wz0 * wy0, g * wz0 * c.fy, g * c.fz * wy0, g * c.fz * c.fy, 1.f - c.fx, c.fx);
     }
 }
 
