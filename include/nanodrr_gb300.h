@@ -411,6 +411,23 @@ NDRR_API int32_t ndrr_pose_so3_fwd(const float* rot, const float* xyz, int32_t p
 
 /* Adjoint for gpose [B, 4, 4]: g_rot, g_xyz [B, 3] per pose (written; the
  * caller sums the rows for a broadcast parameter). */
+/* Local NCC: the same score over every p x p window of [B, C, H, W] float32
+ * images (1 <= p <= min(H, W, NDRR_NCC_PATCH_MOST)): score[b] is the mean
+ * over channels, windows and their pixels. maps: [B, C, 5, H - p + 1,
+ * W - p + 1] float64 window statistics, written by the forward and read by
+ * the adjoint; workspace: ndrr_ncc_patch_workspace_bytes, 8-byte aligned.
+ * The adjoint writes g1 and g2 ([B, C, H, W]; either may be NULL) for the
+ * upstream gradient go [B]. Deterministic. */
+#define NDRR_NCC_PATCH_MOST 128
+#define NDRR_NCC_PATCH_MAPS 5
+NDRR_API int32_t ndrr_ncc_patch_workspace_bytes(int32_t B, int32_t C, int32_t H, int32_t W, int32_t p,
+                                                uint64_t* bytes);
+NDRR_API int32_t ndrr_ncc_patch_fwd(const float* x1, const float* x2, int32_t B, int32_t C, int32_t H, int32_t W,
+                                    int32_t p, float eps, float* score, double* maps, void* workspace,
+                                    uint64_t workspace_bytes, void* stream);
+NDRR_API int32_t ndrr_ncc_patch_bwd(const float* go, const float* x1, const float* x2, const double* maps, int32_t B,
+                                    int32_t C, int32_t H, int32_t W, int32_t p, float* g1, float* g2, void* stream);
+
 NDRR_API int32_t ndrr_pose_so3_bwd(const float* gpose, const float* rot, const float* xyz, int32_t param_rows,
                                    const float* rt_inv, const float* pivot, const float* pivot_inv, int32_t B,
                                    float* g_rot, float* g_xyz, void* stream);

@@ -177,6 +177,10 @@ SIGNATURES: dict[str, tuple] = {
     "ndrr_ncc_bwd": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                       ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
                                       ctypes.c_void_p, ctypes.c_void_p]),
+    "ndrr_ncc_patch_workspace_bytes": (ctypes.c_int32, [ctypes.c_int32] * 5 + [ctypes.POINTER(ctypes.c_uint64)]),
+    "ndrr_ncc_patch_fwd": (ctypes.c_int32, [ctypes.c_void_p] * 2 + [ctypes.c_int32] * 5 + [ctypes.c_float]
+                           + [ctypes.c_void_p] * 3 + [ctypes.c_uint64, ctypes.c_void_p]),
+    "ndrr_ncc_patch_bwd": (ctypes.c_int32, [ctypes.c_void_p] * 4 + [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 3),
     "ndrr_pose_so3_fwd": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p,
                                            ctypes.c_void_p]),

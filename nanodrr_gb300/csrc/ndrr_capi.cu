@@ -473,6 +473,57 @@ int32_t ndrr_texture_create(const float* vol, int32_t D, int32_t H, int32_t W, u
     return ok();
 }
 
+static int32_t ncc_patch_check(int32_t B, int32_t C, int32_t H, int32_t W, int32_t p) {
+    if (B < 1 || C < 1 || H < 1 || W < 1 || p < 1 || p > H || p > W || p > NDRR_NCC_PATCH_MOST)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "local ncc needs B, C >= 1 and 1 <= p <= min(H, W, %d) (got %d, %d, %d, %d, %d)",
+                    NDRR_NCC_PATCH_MOST, B, C, H, W, p);
+    if ((long long)B * C * H * W >= kInt32Max)
+        return fail(NDRR_ERR_LIMIT, "local ncc of %d x %d x %d x %d pixels is too large", B, C, H, W);
+    return NDRR_OK;
+}
+
+int32_t ndrr_ncc_patch_workspace_bytes(int32_t B, int32_t C, int32_t H, int32_t W, int32_t p, uint64_t* bytes) {
+    if (bytes == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "bytes is NULL");
+    const int32_t rc = ncc_patch_check(B, C, H, W, p);
+    if (rc != NDRR_OK) return rc;
+    *bytes = ndrr::ncc_patch_workspace_bytes(B, C, H, W, p);
+    return ok();
+}
+
+int32_t ndrr_ncc_patch_fwd(const float* x1, const float* x2, int32_t B, int32_t C, int32_t H, int32_t W, int32_t p,
+                           float eps, float* score, double* maps, void* workspace, uint64_t workspace_bytes,
+                           void* stream) {
+    const int32_t rc = ncc_patch_check(B, C, H, W, p);
+    if (rc != NDRR_OK) return rc;
+    if (!(eps >= 0.f)) return fail(NDRR_ERR_INVALID_ARGUMENT, "eps must be >= 0");
+    if (x1 == nullptr || x2 == nullptr || score == nullptr || maps == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "x1, x2, score and maps must be non-NULL");
+    if (misaligned(maps, 8) || misaligned(workspace, 8))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "maps and the workspace must be 8-byte aligned");
+    const uint64_t need = ndrr::ncc_patch_workspace_bytes(B, C, H, W, p);
+    if (workspace == nullptr || workspace_bytes < need)
+        return fail(NDRR_ERR_WORKSPACE, "local ncc needs %llu workspace bytes, got %llu", (unsigned long long)need,
+                    (unsigned long long)(workspace ? workspace_bytes : 0));
+    const cudaError_t e = ndrr::launch_ncc_patch_fwd(x1, x2, B, C, H, W, p, eps, score, maps, workspace,
+                                                     reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "local ncc launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_ncc_patch_bwd(const float* go, const float* x1, const float* x2, const double* maps, int32_t B, int32_t C,
+                           int32_t H, int32_t W, int32_t p, float* g1, float* g2, void* stream) {
+    const int32_t rc = ncc_patch_check(B, C, H, W, p);
+    if (rc != NDRR_OK) return rc;
+    if (g1 == nullptr && g2 == nullptr) return ok();
+    if (go == nullptr || x1 == nullptr || x2 == nullptr || maps == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "go, x1, x2 and maps must be non-NULL");
+    if (misaligned(maps, 8)) return fail(NDRR_ERR_INVALID_ARGUMENT, "maps must be 8-byte aligned");
+    const cudaError_t e =
+        ndrr::launch_ncc_patch_bwd(go, x1, x2, maps, B, C, H, W, p, g1, g2, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "local ncc adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
 int32_t ndrr_texture_destroy(uint64_t handle) {
     bool known = false;
     const cudaError_t e = ndrr::texture_destroy(handle, &known);

@@ -54,6 +54,11 @@ cudaError_t launch_ncc_fwd(const float* x1, const float* x2, int B, int P, int N
                            float* stats, void* workspace, cudaStream_t st);
 cudaError_t launch_ncc_bwd(const float* go, const float* x1, const float* x2, const float* stats, int B, int P,
                            int N, float* g1, float* g2, cudaStream_t st);
+uint64_t ncc_patch_workspace_bytes(int B, int C, int H, int W, int p);
+cudaError_t launch_ncc_patch_fwd(const float* x1, const float* x2, int B, int C, int H, int W, int p, float eps,
+                                 float* score, double* maps, void* workspace, cudaStream_t st);
+cudaError_t launch_ncc_patch_bwd(const float* go, const float* x1, const float* x2, const double* maps, int B, int C,
+                                 int H, int W, int p, float* g1, float* g2, cudaStream_t st);
 cudaError_t launch_pose_fwd(const float* rot, const float* xyz, int param_rows, const float* rt_inv,
                             const float* pivot, const float* pivot_inv, int B, float* pose, cudaStream_t st);
 cudaError_t launch_pose_bwd(const float* gpose, const float* rot, const float* xyz, int param_rows,

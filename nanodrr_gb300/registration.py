@@ -151,9 +151,9 @@ def so3_pose(rot: torch.Tensor, xyz: torch.Tensor, rt_inv: torch.Tensor, pivot: 
 class NormalizedCrossCorrelation2d(torch.nn.Module):
     """Score in [-1, 1] per image pair: mean of the product of the two images
     after each is normalised to zero mean and unit variance (+eps), per
-    channel, or per p x p window with `patch_size` (the windows are unfolded
-    into channels first). Computed by the library's NCC kernels
-    (`ndrr_ncc_fwd/bwd`), differentiable in both images."""
+    channel, or per p x p window with `patch_size`. Computed by the library's
+    NCC kernels (`ndrr_ncc_fwd/bwd`, `ndrr_ncc_patch_fwd/bwd` for windows),
+    differentiable in both images."""
 
     def __init__(self, patch_size: int | None = None, eps: float = 1e-7):
         super().__init__()
@@ -161,6 +161,8 @@ class NormalizedCrossCorrelation2d(torch.nn.Module):
         self.eps = eps
 
     def forward(self, x1: torch.Tensor, x2: torch.Tensor) -> torch.Tensor:
+        if self.patch_size is not None and _patch_kernel_takes(x1, x2, self.patch_size):
+            return ncc_patch_score(x1, x2, self.patch_size, float(self.eps))
         if self.patch_size is not None:
             x1, x2 = _to_patches(x1, self.patch_size), _to_patches(x2, self.patch_size)
         if x1.shape != x2.shape:
@@ -239,6 +241,93 @@ def ncc_score(x1: torch.Tensor, x2: torch.Tensor, eps: float = 1e-7) -> torch.Te
     """NCC score [B] of two [B, C, H, W] image batches (reference
     metrics/ncc.py:18-37 without patches)."""
     return _ncc_op(x1, x2, eps)[0]
+
+
+# ----------------------------------------------------------------- local NCC
+_PATCH_MOST = 128  # NDRR_NCC_PATCH_MOST: the window rows one CTA holds in shared memory
+
+
+def _patch_kernel_takes(x1: torch.Tensor, x2: torch.Tensor, p) -> bool:
+    """Whether the window kernels take this pair: float CUDA images of one
+    shape with a p x p window inside them. Everything else (larger windows,
+    empty batches, other types, and the inputs that raise) is unfolded."""
+    return (
+        isinstance(p, int)
+        and x1.is_cuda
+        and x1.device == x2.device
+        and x1.dim() == 4
+        and x1.shape == x2.shape
+        and x1.is_floating_point()
+        and x2.is_floating_point()
+        and 1 <= p <= min(_PATCH_MOST, x1.shape[2], x1.shape[3])
+        and 0 < x1.numel() < 2**31 - 1
+    )
+
+
+@torch.library.custom_op("nanodrr_gb300::ncc_patch", mutates_args=())
+def _ncc_patch_op(x1: torch.Tensor, x2: torch.Tensor, p: int, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
+    """(score [B], window statistics [B, C, 5, H', W'] float64)."""
+    B, C, H, W = x1.shape
+    a, b = x1.float().contiguous(), x2.float().contiguous()
+    score = torch.empty(B, device=x1.device)
+    maps = torch.empty(B, C, 5, H - p + 1, W - p + 1, device=x1.device, dtype=torch.float64)
+    lib = _ffi.load()
+    nb = ctypes.c_uint64(0)
+    _ffi.check(lib.ndrr_ncc_patch_workspace_bytes(B, C, H, W, p, ctypes.byref(nb)), "ndrr_ncc_patch_workspace_bytes")
+    ws = torch.empty(int(nb.value), device=x1.device, dtype=torch.uint8)
+    _ffi.check(lib.ndrr_ncc_patch_fwd(a.data_ptr(), b.data_ptr(), B, C, H, W, p, eps, score.data_ptr(),
+                                      maps.data_ptr(), ws.data_ptr(), ws.numel(),
+                                      torch.cuda.current_stream(x1.device).cuda_stream), "ndrr_ncc_patch_fwd")
+    return score.to(x1.dtype), maps
+
+
+@_ncc_patch_op.register_fake
+def _(x1, x2, p, eps):
+    B, C, H, W = x1.shape
+    return x1.new_empty(B), x1.new_empty(B, C, 5, H - p + 1, W - p + 1, dtype=torch.float64)
+
+
+@torch.library.custom_op("nanodrr_gb300::ncc_patch_bwd", mutates_args=())
+def _ncc_patch_bwd_op(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, maps: torch.Tensor, p: int, need1: bool,
+                      need2: bool) -> tuple[torch.Tensor, torch.Tensor]:
+    B, C, H, W = x1.shape
+    a, b = x1.float().contiguous(), x2.float().contiguous()
+    g1 = torch.empty_like(a) if need1 else a.new_empty(0)
+    g2 = torch.empty_like(b) if need2 else b.new_empty(0)
+    g = go.float().contiguous()
+    _ffi.check(_ffi.load().ndrr_ncc_patch_bwd(g.data_ptr(), a.data_ptr(), b.data_ptr(), maps.data_ptr(), B, C, H, W, p,
+                                              g1.data_ptr() if need1 else None, g2.data_ptr() if need2 else None,
+                                              torch.cuda.current_stream(x1.device).cuda_stream), "ndrr_ncc_patch_bwd")
+    return g1, g2
+
+
+@_ncc_patch_bwd_op.register_fake
+def _(go, x1, x2, maps, p, need1, need2):
+    shape = x1.shape if need1 else (0,)
+    shape2 = x2.shape if need2 else (0,)
+    return x1.new_empty(shape, dtype=torch.float32), x2.new_empty(shape2, dtype=torch.float32)
+
+
+def _ncc_patch_setup(ctx, inputs, output):
+    x1, x2, p, _ = inputs
+    ctx.save_for_backward(x1, x2, output[1])
+    ctx.p = p
+
+
+def _ncc_patch_backward(ctx, g_score, _g_maps):
+    x1, x2, maps = ctx.saved_tensors
+    need1, need2 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+    g1, g2 = _ncc_patch_bwd_op(g_score, x1, x2, maps.contiguous(), ctx.p, need1, need2)
+    return (g1.to(x1.dtype) if need1 else None, g2.to(x2.dtype) if need2 else None, None, None)
+
+
+torch.library.register_autograd("nanodrr_gb300::ncc_patch", _ncc_patch_backward, setup_context=_ncc_patch_setup)
+
+
+def ncc_patch_score(x1: torch.Tensor, x2: torch.Tensor, patch_size: int, eps: float = 1e-7) -> torch.Tensor:
+    """Local NCC score [B]: the mean NCC over every patch_size x patch_size
+    window (reference metrics/ncc.py:18-37, 65-74)."""
+    return _ncc_patch_op(x1, x2, patch_size, eps)[0]
 
 
 def _to_patches(x: torch.Tensor, p: int) -> torch.Tensor:
