@@ -376,6 +376,20 @@ NDRR_API int32_t ndrr_homography_resample_bwd(const float* go, const float* img,
                                               int32_t C, int32_t H, int32_t W, float* gimg, float* ghom,
                                               void* workspace, uint64_t workspace_bytes, void* stream);
 
+/* The reference's `resample(img, k_inv_old, k_inv_new)` whole: hom =
+ * inv(k_old) k_new ([B, 3, 3], written; k_old [n_old, 3, 3] and k_new
+ * [n_new, 3, 3] with n_old, n_new 1 or B) and the warp by it. The adjoint
+ * takes that hom; gimg as above, g_old and g_new ([B, 3, 3] per batch
+ * element, written; both or neither NULL, with the workspace of
+ * ndrr_homography_resample_bwd_workspace_bytes when given). */
+NDRR_API int32_t ndrr_resample_fwd(const float* img, const float* k_old, int32_t n_old, const float* k_new,
+                                   int32_t n_new, int32_t B, int32_t C, int32_t H, int32_t W, float* hom, float* out,
+                                   void* stream);
+NDRR_API int32_t ndrr_resample_bwd(const float* go, const float* img, const float* hom, const float* k_old,
+                                   int32_t n_old, const float* k_new, int32_t n_new, int32_t B, int32_t C, int32_t H,
+                                   int32_t W, float* gimg, float* g_old, float* g_new, void* workspace,
+                                   uint64_t workspace_bytes, void* stream);
+
 /* ---- normalised cross-correlation ------------------------------------------ *
  * Replaces the reference's metrics/ncc.py:8-37 NormalizedCrossCorrelation2d
  * (the image-similarity loss of a registration step). x1, x2: [B, P, N]
@@ -397,20 +411,6 @@ NDRR_API int32_t ndrr_ncc_fwd(const float* x1, const float* x2, int32_t B, int32
 NDRR_API int32_t ndrr_ncc_bwd(const float* go, const float* x1, const float* x2, const float* stats, int32_t B,
                               int32_t P, int32_t N, float* g1, float* g2, void* stream);
 
-/* ---- registration pose ------------------------------------------------------ *
- * Replaces the reference's Registration.pose (registration/registration.py:
- * 64-68 with geometry/se3.py:179-221, "so3_log"): the pose of each batch
- * element is rt_inv @ pivot @ T @ pivot_inv with T = [[R, R xyz], [0, 1]] and
- * R = exp([rot]x) (Rodrigues). rot, xyz: [B or 1, 3] float32 (rows of a
- * single-row parameter are broadcast: pass param_rows 1); rt_inv, pivot,
- * pivot_inv, pose: [B, 4, 4] float32, contiguous. Evaluated in float64, one
- * thread per pose. */
-NDRR_API int32_t ndrr_pose_so3_fwd(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
-                                   const float* pivot, const float* pivot_inv, int32_t B, float* pose,
-                                   void* stream);
-
-/* Adjoint for gpose [B, 4, 4]: g_rot, g_xyz [B, 3] per pose (written; the
- * caller sums the rows for a broadcast parameter). */
 /* Local NCC: the same score over every p x p window of [B, C, H, W] float32
  * images (1 <= p <= min(H, W, NDRR_NCC_PATCH_MOST)): score[b] is the mean
  * over channels, windows and their pixels. maps: [B, C, 5, H - p + 1,
@@ -428,6 +428,20 @@ NDRR_API int32_t ndrr_ncc_patch_fwd(const float* x1, const float* x2, int32_t B,
 NDRR_API int32_t ndrr_ncc_patch_bwd(const float* go, const float* x1, const float* x2, const double* maps, int32_t B,
                                     int32_t C, int32_t H, int32_t W, int32_t p, float* g1, float* g2, void* stream);
 
+/* ---- registration pose ------------------------------------------------------ *
+ * Replaces the reference's Registration.pose (registration/registration.py:
+ * 64-68 with geometry/se3.py:179-221, "so3_log"): the pose of each batch
+ * element is rt_inv @ pivot @ T @ pivot_inv with T = [[R, R xyz], [0, 1]] and
+ * R = exp([rot]x) (Rodrigues). rot, xyz: [B or 1, 3] float32 (rows of a
+ * single-row parameter are broadcast: pass param_rows 1); rt_inv, pivot,
+ * pivot_inv, pose: [B, 4, 4] float32, contiguous. Evaluated in float64, one
+ * thread per pose. */
+NDRR_API int32_t ndrr_pose_so3_fwd(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
+                                   const float* pivot, const float* pivot_inv, int32_t B, float* pose,
+                                   void* stream);
+
+/* Adjoint for gpose [B, 4, 4]: g_rot, g_xyz [B, 3] per pose (written; the
+ * caller sums the rows for a broadcast parameter). */
 NDRR_API int32_t ndrr_pose_so3_bwd(const float* gpose, const float* rot, const float* xyz, int32_t param_rows,
                                    const float* rt_inv, const float* pivot, const float* pivot_inv, int32_t B,
                                    float* g_rot, float* g_xyz, void* stream);

@@ -195,6 +195,10 @@ SIGNATURES: dict[str, tuple] = {
                                                       ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                                       ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                                       ctypes.c_uint64, ctypes.c_void_p]),
+    "ndrr_resample_fwd": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p]
+                          + [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 3),
+    "ndrr_resample_bwd": (ctypes.c_int32, [ctypes.c_void_p] * 4 + [ctypes.c_int32, ctypes.c_void_p]
+                          + [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 4 + [ctypes.c_uint64, ctypes.c_void_p]),
     "ndrr_proposal_last_error": (ctypes.c_char_p, []),
     "ndrr_proposal_dataset": (
         ctypes.c_int32,

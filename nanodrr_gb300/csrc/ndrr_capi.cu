@@ -371,9 +371,56 @@ int32_t ndrr_homography_resample_bwd(const float* go, const float* img, const fl
     if (ghom != nullptr && (workspace == nullptr || workspace_bytes < need))
         return fail(NDRR_ERR_WORKSPACE, "resample adjoint needs %llu workspace bytes, got %llu",
                     (unsigned long long)need, (unsigned long long)(workspace ? workspace_bytes : 0));
-    const cudaError_t e = ndrr::launch_homography_bwd(go, img, hom, B, C, H, W, gimg, ghom,
-                                                      reinterpret_cast<float*>(workspace),
-                                                      reinterpret_cast<cudaStream_t>(stream));
+    const cudaError_t e =
+        ndrr::launch_homography_bwd(go, img, hom, B, C, H, W, gimg, ghom, reinterpret_cast<float*>(workspace), nullptr,
+                                    1, nullptr, 1, nullptr, nullptr, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "resample adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+static int32_t intrinsics_check(const float* k_old, int32_t n_old, const float* k_new, int32_t n_new, int32_t B) {
+    if (k_old == nullptr || k_new == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "k_old and k_new must be non-NULL");
+    if ((n_old != 1 && n_old != B) || (n_new != 1 && n_new != B))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "n_old and n_new must be 1 or B = %d (got %d, %d)", B, n_old, n_new);
+    return NDRR_OK;
+}
+
+int32_t ndrr_resample_fwd(const float* img, const float* k_old, int32_t n_old, const float* k_new, int32_t n_new,
+                          int32_t B, int32_t C, int32_t H, int32_t W, float* hom, float* out, void* stream) {
+    int32_t rc = homography_check(img, hom, B, C, H, W);
+    if (rc != NDRR_OK) return rc;
+    if (B == 0) return ok();
+    rc = intrinsics_check(k_old, n_old, k_new, n_new, B);
+    if (rc != NDRR_OK) return rc;
+    if (out == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "out is NULL");
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    cudaError_t e = ndrr::launch_homography_matrix(k_old, n_old, k_new, n_new, B, hom, st);
+    if (e == cudaSuccess) e = ndrr::launch_homography_fwd(img, hom, B, C, H, W, out, st);
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "resample launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_resample_bwd(const float* go, const float* img, const float* hom, const float* k_old, int32_t n_old,
+                          const float* k_new, int32_t n_new, int32_t B, int32_t C, int32_t H, int32_t W, float* gimg,
+                          float* g_old, float* g_new, void* workspace, uint64_t workspace_bytes, void* stream) {
+    int32_t rc = homography_check(img, hom, B, C, H, W);
+    if (rc != NDRR_OK) return rc;
+    if (B == 0) return ok();
+    if (go == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "go is NULL");
+    if ((g_old == nullptr) != (g_new == nullptr))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "g_old and g_new are both given or both NULL");
+    if (g_old != nullptr) {
+        rc = intrinsics_check(k_old, n_old, k_new, n_new, B);
+        if (rc != NDRR_OK) return rc;
+        const uint64_t need = (uint64_t)B * ndrr::homography_blocks(H, W) * 9 * sizeof(float);
+        if (workspace == nullptr || workspace_bytes < need)
+            return fail(NDRR_ERR_WORKSPACE, "resample adjoint needs %llu workspace bytes, got %llu",
+                        (unsigned long long)need, (unsigned long long)(workspace ? workspace_bytes : 0));
+    }
+    const cudaError_t e = ndrr::launch_homography_bwd(
+        go, img, hom, B, C, H, W, gimg, nullptr, reinterpret_cast<float*>(workspace), g_old ? k_old : nullptr, n_old,
+        k_new, n_new, g_old, g_new, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "resample adjoint launch failed: %s", cudaGetErrorString(e));
     return ok();
 }
@@ -426,53 +473,6 @@ int32_t ndrr_ncc_bwd(const float* go, const float* x1, const float* x2, const fl
     return ok();
 }
 
-static int32_t pose_check(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
-                          const float* pivot, const float* pivot_inv, int32_t B) {
-    if (B < 0) return fail(NDRR_ERR_INVALID_ARGUMENT, "B must be >= 0");
-    if (B == 0) return NDRR_OK;
-    if (!rot || !xyz || !rt_inv || !pivot || !pivot_inv)
-        return fail(NDRR_ERR_INVALID_ARGUMENT, "pose inputs must be non-NULL");
-    if (param_rows != 1 && param_rows != B)
-        return fail(NDRR_ERR_INVALID_ARGUMENT, "param_rows must be 1 or B (%d), got %d", B, param_rows);
-    return NDRR_OK;
-}
-
-int32_t ndrr_pose_so3_fwd(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
-                          const float* pivot, const float* pivot_inv, int32_t B, float* pose, void* stream) {
-    const int32_t rc = pose_check(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B);
-    if (rc != NDRR_OK) return rc;
-    if (B == 0) return ok();
-    if (pose == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "pose is NULL");
-    const cudaError_t e = ndrr::launch_pose_fwd(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, pose,
-                                                reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "pose launch failed: %s", cudaGetErrorString(e));
-    return ok();
-}
-
-int32_t ndrr_pose_so3_bwd(const float* gpose, const float* rot, const float* xyz, int32_t param_rows,
-                          const float* rt_inv, const float* pivot, const float* pivot_inv, int32_t B, float* g_rot,
-                          float* g_xyz, void* stream) {
-    const int32_t rc = pose_check(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B);
-    if (rc != NDRR_OK) return rc;
-    if (B == 0) return ok();
-    if (!gpose || !g_rot || !g_xyz) return fail(NDRR_ERR_INVALID_ARGUMENT, "gpose, g_rot and g_xyz must be non-NULL");
-    const cudaError_t e = ndrr::launch_pose_bwd(gpose, rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, g_rot,
-                                                g_xyz, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "pose adjoint launch failed: %s", cudaGetErrorString(e));
-    return ok();
-}
-
-int32_t ndrr_texture_create(const float* vol, int32_t D, int32_t H, int32_t W, uint64_t* handle, void* stream) {
-    if (vol == nullptr || handle == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "vol and handle must be non-NULL");
-    if (D < 1 || H < 1 || W < 1 || D > 16384 || H > 16384 || W > 16384)
-        return fail(NDRR_ERR_LIMIT, "3-D texture extent %d x %d x %d outside [1, 16384]", D, H, W);
-    unsigned long long h = 0;
-    const cudaError_t e = ndrr::texture_create(vol, D, H, W, &h, reinterpret_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "texture creation failed: %s", cudaGetErrorString(e));
-    *handle = h;
-    return ok();
-}
-
 static int32_t ncc_patch_check(int32_t B, int32_t C, int32_t H, int32_t W, int32_t p) {
     if (B < 1 || C < 1 || H < 1 || W < 1 || p < 1 || p > H || p > W || p > NDRR_NCC_PATCH_MOST)
         return fail(NDRR_ERR_INVALID_ARGUMENT, "local ncc needs B, C >= 1 and 1 <= p <= min(H, W, %d) (got %d, %d, %d, %d, %d)",
@@ -521,6 +521,53 @@ int32_t ndrr_ncc_patch_bwd(const float* go, const float* x1, const float* x2, co
     const cudaError_t e =
         ndrr::launch_ncc_patch_bwd(go, x1, x2, maps, B, C, H, W, p, g1, g2, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "local ncc adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+static int32_t pose_check(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
+                          const float* pivot, const float* pivot_inv, int32_t B) {
+    if (B < 0) return fail(NDRR_ERR_INVALID_ARGUMENT, "B must be >= 0");
+    if (B == 0) return NDRR_OK;
+    if (!rot || !xyz || !rt_inv || !pivot || !pivot_inv)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "pose inputs must be non-NULL");
+    if (param_rows != 1 && param_rows != B)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "param_rows must be 1 or B (%d), got %d", B, param_rows);
+    return NDRR_OK;
+}
+
+int32_t ndrr_pose_so3_fwd(const float* rot, const float* xyz, int32_t param_rows, const float* rt_inv,
+                          const float* pivot, const float* pivot_inv, int32_t B, float* pose, void* stream) {
+    const int32_t rc = pose_check(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B);
+    if (rc != NDRR_OK) return rc;
+    if (B == 0) return ok();
+    if (pose == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "pose is NULL");
+    const cudaError_t e = ndrr::launch_pose_fwd(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, pose,
+                                                reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "pose launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_pose_so3_bwd(const float* gpose, const float* rot, const float* xyz, int32_t param_rows,
+                          const float* rt_inv, const float* pivot, const float* pivot_inv, int32_t B, float* g_rot,
+                          float* g_xyz, void* stream) {
+    const int32_t rc = pose_check(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B);
+    if (rc != NDRR_OK) return rc;
+    if (B == 0) return ok();
+    if (!gpose || !g_rot || !g_xyz) return fail(NDRR_ERR_INVALID_ARGUMENT, "gpose, g_rot and g_xyz must be non-NULL");
+    const cudaError_t e = ndrr::launch_pose_bwd(gpose, rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, g_rot,
+                                                g_xyz, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "pose adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_texture_create(const float* vol, int32_t D, int32_t H, int32_t W, uint64_t* handle, void* stream) {
+    if (vol == nullptr || handle == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "vol and handle must be non-NULL");
+    if (D < 1 || H < 1 || W < 1 || D > 16384 || H > 16384 || W > 16384)
+        return fail(NDRR_ERR_LIMIT, "3-D texture extent %d x %d x %d outside [1, 16384]", D, H, W);
+    unsigned long long h = 0;
+    const cudaError_t e = ndrr::texture_create(vol, D, H, W, &h, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "texture creation failed: %s", cudaGetErrorString(e));
+    *handle = h;
     return ok();
 }
 

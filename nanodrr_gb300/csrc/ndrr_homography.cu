@@ -138,15 +138,116 @@ __global__ void __launch_bounds__(kHomBlock) homography_bwd_kernel(const float* 
     }
 }
 
-// Per-batch fixed-order sum of the CTA partials into ghom [B, 3, 3].
-__global__ void __launch_bounds__(32) homography_reduce_kernel(const float* __restrict__ partials, int nblk,
-                                                               float* __restrict__ ghom) {
-    const int b = blockIdx.x;
-    const int j = threadIdx.x;
+// Per-batch fixed-order sum of the CTA partials into ghom [B, 3, 3]: each
+// thread takes a strided share in double, then a shuffle tree (one thread per
+// entry walking all 1024 partials of a 512^2 image took 22 us).
+// With `k_old`, ghom is not written but chained to the two inverse intrinsics
+// of H = inv(k_old) k_new (float64): g_new = A^T g, g_old = -A^T (g k_new^T)
+// A^T with A = inv(k_old).
+constexpr int kHomReduce = 128;
+
+__device__ __forceinline__ void inverse3(const double (&m)[9], double (&r)[9]) {
+    r[0] = m[4] * m[8] - m[5] * m[7];
+    r[1] = m[2] * m[7] - m[1] * m[8];
+    r[2] = m[1] * m[5] - m[2] * m[4];
+    r[3] = m[5] * m[6] - m[3] * m[8];
+    r[4] = m[0] * m[8] - m[2] * m[6];
+    r[5] = m[2] * m[3] - m[0] * m[5];
+    r[6] = m[3] * m[7] - m[4] * m[6];
+    r[7] = m[1] * m[6] - m[0] * m[7];
+    r[8] = m[0] * m[4] - m[1] * m[3];
+    const double inv = 1.0 / (m[0] * r[0] + m[1] * r[3] + m[2] * r[6]);
+    for (int i = 0; i < 9; ++i) r[i] *= inv;
+}
+
+__global__ void __launch_bounds__(kHomReduce) homography_reduce_kernel(const float* __restrict__ partials, int nblk,
+                                                                       float* __restrict__ ghom,
+                                                                       const float* __restrict__ k_old, int n_old,
+                                                                       const float* __restrict__ k_new, int n_new,
+                                                                       float* __restrict__ g_old,
+                                                                       float* __restrict__ g_new) {
+    __shared__ double red[kHomReduce / 32][9];
+    __shared__ double g[9], A[9], t[9];
+    const int b = blockIdx.x, j = threadIdx.x;
+    double s[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) s[k] = 0.0;
+    for (int i = threadIdx.x; i < nblk; i += kHomReduce)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) s[k] += (double)partials[((size_t)b * nblk + i) * 9 + k];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        if ((j & 31) == 0) red[j >> 5][k] = s[k];
+    }
+    __syncthreads();
+    if (j < 9) {
+        double v = red[0][j];
+        for (int w = 1; w < kHomReduce / 32; ++w) v += red[w][j];
+        g[j] = v;
+        if (ghom != nullptr) ghom[(size_t)b * 9 + j] = (float)v;
+    }
+    if (k_old == nullptr) return;
+    const float* ko = k_old + (n_old == 1 ? 0 : (size_t)b * 9);
+    const float* kn = k_new + (n_new == 1 ? 0 : (size_t)b * 9);
+    if (j == 32) {
+        double m[9], r[9];
+        for (int i = 0; i < 9; ++i) m[i] = (double)ko[i];
+        inverse3(m, r);
+        for (int i = 0; i < 9; ++i) A[i] = r[i];
+    }
+    __syncthreads();
     if (j >= 9) return;
-    float s = 0.f;
-    for (int k = 0; k < nblk; ++k) s += partials[((size_t)b * nblk + k) * 9 + j];
-    ghom[(size_t)b * 9 + j] = s;
+    const int r = j / 3, c = j % 3;
+    const unsigned lanes = 0x1ffu;  // the nine threads that go on
+    double v = 0.0, u = 0.0;
+    for (int i = 0; i < 3; ++i) {
+        v += A[3 * i + r] * g[3 * i + c];                   // A^T g
+        u += g[3 * r + i] * (double)kn[3 * c + i];          // g k_new^T
+    }
+    g_new[(size_t)b * 9 + j] = (float)v;
+    t[j] = u;
+    __syncwarp(lanes);
+    double w = 0.0;
+    for (int i = 0; i < 3; ++i) w += A[3 * i + r] * t[3 * i + c];  // A^T (g k_new^T)
+    __syncwarp(lanes);
+    t[j] = w;
+    __syncwarp(lanes);
+    double x = 0.0;
+    for (int i = 0; i < 3; ++i) x += t[3 * r + i] * A[3 * c + i];  // ... A^T
+    g_old[(size_t)b * 9 + j] = (float)-x;
+}
+
+// H = inv(k_old) k_new per batch element, one thread each: the float32
+// cofactor inverse and products in the order of the tensor expression
+// (homography.py::_inv3, mm_small), so the homography is bitwise its.
+__global__ void __launch_bounds__(32) homography_matrix_kernel(const float* __restrict__ k_old, int n_old,
+                                                               const float* __restrict__ k_new, int n_new, int B,
+                                                               float* __restrict__ hom) {
+    const int t = blockIdx.x * 32 + threadIdx.x;
+    if (t >= B) return;
+    const float* m = k_old + (n_old == 1 ? 0 : (size_t)t * 9);
+    const float* q = k_new + (n_new == 1 ? 0 : (size_t)t * 9);
+    const float a = m[0], b = m[1], c = m[2], d = m[3], e = m[4], f = m[5], g = m[6], h = m[7], i = m[8];
+    auto minor = [](float w, float x, float y, float z) { return __fsub_rn(__fmul_rn(w, x), __fmul_rn(y, z)); };
+    float co[9] = {minor(e, i, f, h), minor(c, h, b, i), minor(b, f, c, e), minor(f, g, d, i), minor(a, i, c, g),
+                   minor(c, d, a, f), minor(d, h, e, g), minor(b, g, a, h), minor(a, e, b, d)};
+    const float det = __fadd_rn(__fadd_rn(__fmul_rn(a, co[0]), __fmul_rn(b, co[3])), __fmul_rn(c, co[6]));
+#pragma unroll
+    for (int k = 0; k < 9; ++k) co[k] = __fdiv_rn(co[k], det);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            hom[(size_t)t * 9 + 3 * r + k] =
+                __fadd_rn(__fadd_rn(__fmul_rn(co[3 * r], q[k]), __fmul_rn(co[3 * r + 1], q[3 + k])),
+                          __fmul_rn(co[3 * r + 2], q[6 + k]));
+}
+
+cudaError_t launch_homography_matrix(const float* k_old, int n_old, const float* k_new, int n_new, int B, float* hom,
+                                     cudaStream_t st) {
+    homography_matrix_kernel<<<(B + 31) / 32, 32, 0, st>>>(k_old, n_old, k_new, n_new, B, hom);
+    return cudaGetLastError();
 }
 
 int homography_blocks(int H, int W) { return (H * W + kHomBlock - 1) / kHomBlock; }
@@ -159,13 +260,15 @@ cudaError_t launch_homography_fwd(const float* img, const float* hom, int B, int
 }
 
 cudaError_t launch_homography_bwd(const float* go, const float* img, const float* hom, int B, int C, int H, int W,
-                                  float* gimg, float* ghom, float* partials, cudaStream_t st) {
+                                  float* gimg, float* ghom, float* partials, const float* k_old, int n_old,
+                                  const float* k_new, int n_new, float* g_old, float* g_new, cudaStream_t st) {
     const int nblk = homography_blocks(H, W);
     const dim3 grid((unsigned)nblk, (unsigned)B);
-    homography_bwd_kernel<<<grid, kHomBlock, 0, st>>>(go, img, hom, gimg, ghom ? partials : nullptr, C, H, W);
+    const bool reduce = ghom != nullptr || k_old != nullptr;
+    homography_bwd_kernel<<<grid, kHomBlock, 0, st>>>(go, img, hom, gimg, reduce ? partials : nullptr, C, H, W);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || ghom == nullptr) return e;
-    homography_reduce_kernel<<<B, 32, 0, st>>>(partials, nblk, ghom);
+    if (e != cudaSuccess || !reduce) return e;
+    homography_reduce_kernel<<<B, kHomReduce, 0, st>>>(partials, nblk, ghom, k_old, n_old, k_new, n_new, g_old, g_new);
     return cudaGetLastError();
 }
 

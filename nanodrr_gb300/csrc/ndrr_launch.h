@@ -67,7 +67,10 @@ cudaError_t launch_pose_bwd(const float* gpose, const float* rot, const float* x
 cudaError_t launch_homography_fwd(const float* img, const float* hom, int B, int C, int H, int W, float* out,
                                   cudaStream_t st);
 cudaError_t launch_homography_bwd(const float* go, const float* img, const float* hom, int B, int C, int H, int W,
-                                  float* gimg, float* ghom, float* partials, cudaStream_t st);
+                                  float* gimg, float* ghom, float* partials, const float* k_old, int n_old,
+                                  const float* k_new, int n_new, float* g_old, float* g_new, cudaStream_t st);
+cudaError_t launch_homography_matrix(const float* k_old, int n_old, const float* k_new, int n_new, int B, float* hom,
+                                     cudaStream_t st);
 cudaError_t launch_batched(const ndrr_batch_args& a, bool backward, int sm_count, cudaStream_t st);
 cudaError_t device_flags(unsigned* out, bool clear);
 cudaError_t launch_camera_rays(const float* k_inv, int n_k, const float* sdd, int n_s, int B, int height, int width,

@@ -56,3 +56,32 @@ def test_resample_homography_gradient_is_deterministic_and_rejects_bad_input():
     assert torch.equal(grads[0], grads[1])
     with pytest.raises(ValueError, match="float32"):
         nd.resample(img.double(), ko.detach().double(), kn.double())
+
+
+@pytest.mark.parametrize("n_old,n_new", [(1, 1), (4, 1), (1, 4), (4, 4)])
+@pytest.mark.parametrize("shape", [(4, 1, 2, 2), (4, 3, 33, 47), (4, 2, 190, 150)])
+def test_resample_equals_the_warp_by_the_tensor_homography(shape, n_old, n_new):
+    """One launch per direction against the composed expression: shared and
+    per-image cameras, one block and several, every gradient."""
+    from nanodrr_gb300.geometry import mm_small
+    from nanodrr_gb300.homography import _inv3, homography_resample
+
+    g = torch.Generator().manual_seed(n_old + 2 * n_new)
+    B, _, H, W = shape
+    k = nd.make_k_inv(900.0, 1.3, 1.2, 0.4, -0.3, H, W)
+    jitter = lambda n: 1 + 0.01 * torch.rand(n, 3, 3, generator=g)  # noqa: E731
+    cams = [(k * jitter(n)).to(DEV) for n in (n_old, n_new)]
+    img, go = (torch.rand(shape, generator=g).to(DEV) for _ in range(2))
+    got, want = [], []
+    for res, composed in ((got, False), (want, True)):
+        leaves = [t.clone().requires_grad_(True) for t in (img, *cams)]
+        if composed:
+            out = homography_resample(leaves[0], mm_small(_inv3(leaves[1]), leaves[2]).expand(B, 3, 3).contiguous())
+        else:
+            out = nd.resample(*leaves)
+        out.backward(go)
+        res += [out.detach()] + [t.grad for t in leaves]
+    # the same homography; the camera gradients differ by the float32
+    # rounding of the composed chain through the inverse
+    for a, b, tol in zip(got, want, (1e-6, 1e-5, 1e-4, 1e-4)):
+        assert a.shape == b.shape and rel_maxabs(a, b) < tol
