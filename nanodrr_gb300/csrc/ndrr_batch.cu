@@ -106,29 +106,27 @@ __global__ void __launch_bounds__(256, 4) batched_bwd_kernel(const BatchParams b
     }
 }
 
-// Per-request fixed-order sum of its tile partials (one CTA per request).
+// Per-request fixed-order sum of its tile partials (one CTA per request and
+// term).
 __global__ void __launch_bounds__(256) batched_reduce_kernel(const BatchParams bp, int gcam) {
-    __shared__ float red[8][16];
-    const int r = blockIdx.x;
+    __shared__ float red[8];
+    const int r = blockIdx.x, j = blockIdx.y;
     const ndrr_request& q = bp.req[r];
+    if (j >= 12 && !(gcam && !q.src_per_ray)) return;
     const int t0 = __ldg(bp.off + r), t1 = __ldg(bp.off + r + 1);
-    const bool shared_src = gcam && !q.src_per_ray;
-    const int nterms = shared_src ? 15 : 12;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int j = 0; j < nterms; ++j) {
-        float v = 0.f;
-        for (int t = t0 + tid; t < t1; t += blockDim.x) v += bp.partials[(size_t)t * kPartialStride + j];
-        v = warp_sum(v);
-        if (lane == 0) red[warp][j] = v;
-    }
+    float v = 0.f;
+    for (int t = t0 + tid; t < t1; t += blockDim.x) v += bp.partials[(size_t)t * kPartialStride + j];
+    v = warp_sum(v);
+    if (lane == 0) red[warp] = v;
     __syncthreads();
-    if (tid < nterms) {
+    if (tid == 0) {
         float sum = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += red[w][tid];
-        if (tid < 12)
-            q.gM[tid] = sum;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += red[w];
+        if (j < 12)
+            q.gM[j] = sum;
         else
-            q.gsrc[tid - 12] = sum;
+            q.gsrc[j - 12] = sum;
     }
 }
 
@@ -203,7 +201,7 @@ cudaError_t launch_batched(const ndrr_batch_args& a, bool backward, int sm_count
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    batched_reduce_kernel<<<a.n_requests, 256, 0, st>>>(bp, gcam ? 1 : 0);
+    batched_reduce_kernel<<<dim3((unsigned)a.n_requests, gcam ? 15 : 12), 256, 0, st>>>(bp, gcam ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -4,7 +4,7 @@
 //   pose = rt_inv @ pivot @ T @ pivot_inv,  T = [[R, R xyz], [0, 1]],
 //   R = exp([v]x) = I + a K + b K^2,  K = [v]x,
 //   a = sin(t) / t,  b = (1 - cos t) / t^2,  t = |v|,
-// and its adjoint to (v, xyz). One thread per pose in float64: the handful
+// and its adjoint to (v, xyz). One warp per pose in float64: the handful
 // of 4x4 products replace about thirty elementwise torch launches per
 // direction, and float64 keeps b and the derivatives of a and b accurate
 // where float32 cancels (t between 1e-4 and 1e-2).
@@ -34,42 +34,60 @@ __device__ __forceinline__ void rodrigues_coefficients(double t2, double& a, dou
     }
 }
 
-struct PoseTerms {
-    double v[3], x[3];
+// One warp per pose: lane l < 16 owns entry (l / 4, l % 4) of every 4x4
+// matrix, exchanged through shared memory. What bounds these kernels is the
+// fp64 pipe, which takes a warp instruction every 16 cycles whatever its
+// active lanes, and the chain of dependent operations: one thread per pose
+// issued about 400 of them (12 and 14 us); 16 lanes issue 40 and 80 (3.7 and
+// 5.3 us).
+struct PoseShared {
+    double A[16], P[16], C[16], G[16], X[16], Y[16];
     double K[3][3], K2[3][3], R[3][3];
-    double a, b, ca, cb;
 };
 
-__device__ __forceinline__ void pose_terms(const float* rot, const float* xyz, int row, PoseTerms& q) {
-    for (int i = 0; i < 3; ++i) {
-        q.v[i] = (double)rot[row * 3 + i];
-        q.x[i] = (double)xyz[row * 3 + i];
+struct PoseCoef {
+    double v[3], x[3], a, b, ca, cb;
+};
+
+__device__ __forceinline__ double mul_entry(const double* A, const double* B, int i, int j) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s += A[4 * i + k] * B[4 * k + j];
+    return s;
+}
+
+// Loads the pose's matrices, forms K, K^2, R and leaves rt_inv @ pivot in X.
+__device__ __forceinline__ void pose_setup(PoseShared& q, PoseCoef& c, const float* rot, const float* xyz, int row,
+                                           const float* rt_inv, const float* pivot, const float* pivot_inv, int b,
+                                           int l) {
+    const int i = l >> 2, j = l & 3;
+    if (l < 16) {
+        q.A[l] = (double)rt_inv[(size_t)b * 16 + l];
+        q.P[l] = (double)pivot[(size_t)b * 16 + l];
+        q.C[l] = (double)pivot_inv[(size_t)b * 16 + l];
     }
-    const double vx = q.v[0], vy = q.v[1], vz = q.v[2];
-    const double K[3][3] = {{0.0, -vz, vy}, {vz, 0.0, -vx}, {-vy, vx, 0.0}};
-    rodrigues_coefficients(vx * vx + vy * vy + vz * vz, q.a, q.b, q.ca, q.cb);
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-            q.K[i][j] = K[i][j];
-            double s = 0.0;
-            for (int k = 0; k < 3; ++k) s += K[i][k] * K[k][j];
-            q.K2[i][j] = s;
-            q.R[i][j] = (i == j ? 1.0 : 0.0) + q.a * K[i][j] + q.b * s;
-        }
-}
-
-__device__ __forceinline__ void load44(const float* m, double (&o)[4][4]) {
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) o[i][j] = (double)m[i * 4 + j];
-}
-
-__device__ __forceinline__ void mul44(const double (&A)[4][4], const double (&B)[4][4], double (&C)[4][4]) {
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s += A[i][k] * B[k][j];
-            C[i][j] = s;
-        }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        c.v[k] = (double)rot[row * 3 + k];
+        c.x[k] = (double)xyz[row * 3 + k];
+    }
+    const double vx = c.v[0], vy = c.v[1], vz = c.v[2];
+    rodrigues_coefficients(vx * vx + vy * vy + vz * vz, c.a, c.b, c.ca, c.cb);
+    const bool rotation = l < 16 && i < 3 && j < 3;
+    if (rotation) {  // K = [v]x: row i has -v at the axis after i's next, v at its next
+        const int n = 3 - i - j;  // the third axis (i != j)
+        q.K[i][j] = i == j ? 0.0 : ((j - i + 3) % 3 == 1 ? -1.0 : 1.0) * c.v[n];
+    }
+    __syncwarp();
+    if (rotation) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s += q.K[i][k] * q.K[k][j];
+        q.K2[i][j] = s;
+        q.R[i][j] = (i == j ? 1.0 : 0.0) + c.a * q.K[i][j] + c.b * s;
+    }
+    if (l < 16) q.X[l] = mul_entry(q.A, q.P, i, j);
+    __syncwarp();
 }
 
 __global__ void __launch_bounds__(kPoseBlock) pose_so3_fwd_kernel(const float* __restrict__ rot,
@@ -78,26 +96,25 @@ __global__ void __launch_bounds__(kPoseBlock) pose_so3_fwd_kernel(const float* _
                                                                   const float* __restrict__ pivot,
                                                                   const float* __restrict__ pivot_inv, int B,
                                                                   float* __restrict__ pose) {
-    const int b = blockIdx.x * kPoseBlock + threadIdx.x;
-    if (b >= B) return;
-    PoseTerms q;
-    pose_terms(rot, xyz, param_rows == 1 ? 0 : b, q);
-    double T[4][4], A[4][4], P[4][4], C[4][4], AT[4][4], out[4][4];
-    for (int i = 0; i < 3; ++i) {
-        for (int j = 0; j < 3; ++j) T[i][j] = q.R[i][j];
-        T[i][3] = q.R[i][0] * q.x[0] + q.R[i][1] * q.x[1] + q.R[i][2] * q.x[2];
+    __shared__ PoseShared sh[kPoseBlock / 32];
+    const int l = threadIdx.x & 31, b = blockIdx.x * (kPoseBlock / 32) + (threadIdx.x >> 5);
+    if (b >= B) return;  // whole warps
+    PoseShared& q = sh[threadIdx.x >> 5];
+    PoseCoef c;
+    pose_setup(q, c, rot, xyz, param_rows == 1 ? 0 : b, rt_inv, pivot, pivot_inv, b, l);
+    const int i = l >> 2, j = l & 3;
+    if (l < 16) {
+        if (i == 3)
+            q.Y[l] = j == 3 ? 1.0 : 0.0;
+        else
+            q.Y[l] = j < 3 ? q.R[i][j] : q.R[i][0] * c.x[0] + q.R[i][1] * c.x[1] + q.R[i][2] * c.x[2];
     }
-    T[3][0] = T[3][1] = T[3][2] = 0.0;
-    T[3][3] = 1.0;
-    load44(rt_inv + (size_t)b * 16, A);
-    load44(pivot + (size_t)b * 16, P);
-    load44(pivot_inv + (size_t)b * 16, C);
-    double AP[4][4];
-    mul44(A, P, AP);
-    mul44(AP, T, AT);
-    mul44(AT, C, out);
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) pose[(size_t)b * 16 + i * 4 + j] = (float)out[i][j];
+    __syncwarp();
+    const double at = l < 16 ? mul_entry(q.X, q.Y, i, j) : 0.0;
+    __syncwarp();
+    if (l < 16) q.X[l] = at;
+    __syncwarp();
+    if (l < 16) pose[(size_t)b * 16 + l] = (float)mul_entry(q.X, q.C, i, j);
 }
 
 // gT = (rt_inv pivot)^T gpose pivot_inv^T; gR = gT[:3, :3] + gT[:3, 3] xyz^T,
@@ -112,64 +129,70 @@ __global__ void __launch_bounds__(kPoseBlock) pose_so3_bwd_kernel(const float* _
                                                                   const float* __restrict__ pivot_inv, int B,
                                                                   float* __restrict__ g_rot,
                                                                   float* __restrict__ g_xyz) {
-    const int b = blockIdx.x * kPoseBlock + threadIdx.x;
-    if (b >= B) return;
-    PoseTerms q;
-    pose_terms(rot, xyz, param_rows == 1 ? 0 : b, q);
-    double A[4][4], P[4][4], C[4][4], G[4][4], AP[4][4], L[4][4], gT[4][4];
-    load44(rt_inv + (size_t)b * 16, A);
-    load44(pivot + (size_t)b * 16, P);
-    load44(pivot_inv + (size_t)b * 16, C);
-    load44(gpose + (size_t)b * 16, G);
-    mul44(A, P, AP);
-    // L = AP^T G, gT = L C^T
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s += AP[k][i] * G[k][j];
-            L[i][j] = s;
-        }
-    for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s += L[i][k] * C[j][k];
-            gT[i][j] = s;
-        }
-    double gR[3][3], sK = 0.0, sK2 = 0.0;
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-            gR[i][j] = gT[i][j] + gT[i][3] * q.x[j];
-            sK += gR[i][j] * q.K[i][j];
-            sK2 += gR[i][j] * q.K2[i][j];
-        }
-    for (int j = 0; j < 3; ++j)
-        g_xyz[(size_t)b * 3 + j] = (float)(q.R[0][j] * gT[0][3] + q.R[1][j] * gT[1][3] + q.R[2][j] * gT[2][3]);
-    // H = gR K^T + K^T gR
-    double H[3][3];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 3; ++k) s += gR[i][k] * q.K[j][k] + q.K[k][i] * gR[k][j];
-            H[i][j] = s;
-        }
-    const double radial = q.ca * sK + q.cb * sK2;
-    const double vr[3] = {gR[2][1] - gR[1][2], gR[0][2] - gR[2][0], gR[1][0] - gR[0][1]};
-    const double vh[3] = {H[2][1] - H[1][2], H[0][2] - H[2][0], H[1][0] - H[0][1]};
-    for (int i = 0; i < 3; ++i) g_rot[(size_t)b * 3 + i] = (float)(radial * q.v[i] + q.a * vr[i] + q.b * vh[i]);
+    __shared__ PoseShared sh[kPoseBlock / 32];
+    const int l = threadIdx.x & 31, b = blockIdx.x * (kPoseBlock / 32) + (threadIdx.x >> 5);
+    if (b >= B) return;  // whole warps
+    PoseShared& q = sh[threadIdx.x >> 5];
+    PoseCoef c;
+    if (l < 16) q.G[l] = (double)gpose[(size_t)b * 16 + l];
+    pose_setup(q, c, rot, xyz, param_rows == 1 ? 0 : b, rt_inv, pivot, pivot_inv, b, l);
+    const int i = l >> 2, j = l & 3;
+    if (l < 16) {  // L = (rt_inv pivot)^T gpose
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s += q.X[4 * k + i] * q.G[4 * k + j];
+        q.Y[l] = s;
+    }
+    __syncwarp();
+    if (l < 16) {  // gT = L pivot_inv^T
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s += q.Y[4 * i + k] * q.C[4 * j + k];
+        q.G[l] = s;
+    }
+    __syncwarp();
+    const bool rotation = l < 16 && i < 3 && j < 3;
+    if (rotation) q.P[3 * i + j] = q.G[l] + q.G[4 * i + 3] * c.x[j];  // gR
+    if (l < 3)
+        g_xyz[(size_t)b * 3 + l] = (float)(q.R[0][l] * q.G[3] + q.R[1][l] * q.G[7] + q.R[2][l] * q.G[11]);
+    __syncwarp();
+    const double* gR = q.P;
+    double sK = 0.0, sK2 = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        sK += gR[k] * q.K[k / 3][k % 3];
+        sK2 += gR[k] * q.K2[k / 3][k % 3];
+    }
+    if (rotation) {  // H = gR K^T + K^T gR
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s += gR[3 * i + k] * q.K[j][k] + q.K[k][i] * gR[3 * k + j];
+        q.A[3 * i + j] = s;
+    }
+    __syncwarp();
+    if (l < 3) {
+        const double* H = q.A;
+        const int u = (l + 2) % 3, w = (l + 1) % 3;  // vee(G)_l = G[u][w] - G[w][u]
+        const double radial = c.ca * sK + c.cb * sK2;
+        const double vr = gR[3 * u + w] - gR[3 * w + u], vh = H[3 * u + w] - H[3 * w + u];
+        const double v = l == 0 ? c.v[0] : (l == 1 ? c.v[1] : c.v[2]);
+        g_rot[(size_t)b * 3 + l] = (float)(radial * v + c.a * vr + c.b * vh);
+    }
 }
+
+static unsigned pose_grid(int B) { return (unsigned)((B + kPoseBlock / 32 - 1) / (kPoseBlock / 32)); }
 
 cudaError_t launch_pose_fwd(const float* rot, const float* xyz, int param_rows, const float* rt_inv,
                             const float* pivot, const float* pivot_inv, int B, float* pose, cudaStream_t st) {
-    pose_so3_fwd_kernel<<<(B + kPoseBlock - 1) / kPoseBlock, kPoseBlock, 0, st>>>(rot, xyz, param_rows, rt_inv,
-                                                                                  pivot, pivot_inv, B, pose);
+    pose_so3_fwd_kernel<<<pose_grid(B), kPoseBlock, 0, st>>>(rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, pose);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pose_bwd(const float* gpose, const float* rot, const float* xyz, int param_rows,
                             const float* rt_inv, const float* pivot, const float* pivot_inv, int B, float* g_rot,
                             float* g_xyz, cudaStream_t st) {
-    pose_so3_bwd_kernel<<<(B + kPoseBlock - 1) / kPoseBlock, kPoseBlock, 0, st>>>(
-        gpose, rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B, g_rot, g_xyz);
+    pose_so3_bwd_kernel<<<pose_grid(B), kPoseBlock, 0, st>>>(gpose, rot, xyz, param_rows, rt_inv, pivot, pivot_inv, B,
+                                                             g_rot, g_xyz);
     return cudaGetLastError();
 }
 
