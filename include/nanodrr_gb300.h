@@ -550,6 +550,29 @@ NDRR_API int32_t ndrr_camera_rays(const float* k_inv, int32_t n_k, const float* 
                                   int32_t height, int32_t width, int32_t orthographic, float* src, float* tgt,
                                   void* stream);
 
+/* The ray set-up of a render call, one launch: src and tgt as above for every
+ * element of `batch` (n_k and n_s each 1 or batch) and step [batch,
+ * height*width] = |tgt - src| / (n_samples - 1). The adjoint takes the
+ * gradients of the three (each may be NULL: zero) and writes g_k [batch, 3,
+ * 3] and g_sdd [batch] per batch element (the caller sums them for a shared
+ * camera); deterministic. */
+NDRR_API int32_t ndrr_ray_setup(const float* k_inv, int32_t n_k, const float* sdd, int32_t n_s, int32_t batch,
+                                int32_t height, int32_t width, int32_t orthographic, int32_t n_samples, float* src,
+                                float* tgt, float* step, void* stream);
+NDRR_API int32_t ndrr_ray_setup_bwd_workspace_bytes(int32_t batch, int32_t height, int32_t width, uint64_t* bytes);
+NDRR_API int32_t ndrr_ray_setup_bwd(const float* k_inv, int32_t n_k, const float* sdd, int32_t n_s, int32_t batch,
+                                    int32_t height, int32_t width, int32_t orthographic, int32_t n_samples,
+                                    const float* gsrc, const float* gtgt, const float* gstep, float* g_k,
+                                    float* g_sdd, void* workspace, uint64_t workspace_bytes, void* stream);
+
+/* The camera -> voxel affine M [batch, 3, 4] = (w2v @ rt)[:3] (w2v [4, 4],
+ * rt [batch, 4, 4]) in float32 and, when M_lo is not NULL, the remainder of
+ * the float64 product (ndrr_raymarch_args.M_lo). The adjoint writes g_rt
+ * [batch, 4, 4] for gM [batch, 3, 4]. */
+NDRR_API int32_t ndrr_camera_affine(const float* w2v, const float* rt, int32_t batch, float* M, float* M_lo,
+                                    void* stream);
+NDRR_API int32_t ndrr_camera_affine_bwd(const float* w2v, const float* gM, int32_t batch, float* g_rt, void* stream);
+
 /* ---- measurement ------------------------------------------------------------ *
  * Kernel timing hook: while set, the calling thread's ray-march entry points
  * record `start` (a cudaEvent_t) on their stream just before each ray-march

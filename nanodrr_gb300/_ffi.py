@@ -157,6 +157,13 @@ SIGNATURES: dict[str, tuple] = {
     "ndrr_camera_rays": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
                                           ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                           ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
+    "ndrr_ray_setup": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p] + [ctypes.c_int32] * 6
+                       + [ctypes.c_void_p] * 4),
+    "ndrr_ray_setup_bwd_workspace_bytes": (ctypes.c_int32, [ctypes.c_int32] * 3 + [ctypes.POINTER(ctypes.c_uint64)]),
+    "ndrr_ray_setup_bwd": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p] + [ctypes.c_int32] * 6
+                           + [ctypes.c_void_p] * 6 + [ctypes.c_uint64, ctypes.c_void_p]),
+    "ndrr_camera_affine": (ctypes.c_int32, [ctypes.c_void_p] * 2 + [ctypes.c_int32] + [ctypes.c_void_p] * 3),
+    "ndrr_camera_affine_bwd": (ctypes.c_int32, [ctypes.c_void_p] * 2 + [ctypes.c_int32] + [ctypes.c_void_p] * 2),
     "ndrr_hu_to_mu": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_float, ctypes.c_float,
                                        ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p]),
     "ndrr_set_kernel_events": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_void_p]),

@@ -657,6 +657,77 @@ int32_t ndrr_camera_rays(const float* k_inv, int32_t n_k, const float* sdd, int3
     return ok();
 }
 
+static int32_t ray_setup_check(const float* k_inv, int32_t n_k, const float* sdd, int32_t n_s, int32_t batch,
+                               int32_t height, int32_t width, int32_t n_samples) {
+    if (k_inv == nullptr || sdd == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "k_inv and sdd must be non-NULL");
+    if (height < 1 || width < 1 || batch < 1 || n_samples < 2)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "height, width and batch must be >= 1 and n_samples >= 2 (got %d, %d, %d, %d)",
+                    height, width, batch, n_samples);
+    if ((n_k != 1 && n_k != batch) || (n_s != 1 && n_s != batch))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "n_k and n_s must be 1 or the batch %d (got %d, %d)", batch, n_k, n_s);
+    if ((long long)batch * height * width * 3 >= (1LL << 31))
+        return fail(NDRR_ERR_LIMIT, "batch x pixels x 3 exceeds int32 indexing");
+    if (batch > 65535) return fail(NDRR_ERR_LIMIT, "the ray set-up takes at most 65535 poses (got %d)", batch);
+    return NDRR_OK;
+}
+
+int32_t ndrr_ray_setup(const float* k_inv, int32_t n_k, const float* sdd, int32_t n_s, int32_t batch, int32_t height,
+                       int32_t width, int32_t orthographic, int32_t n_samples, float* src, float* tgt, float* step,
+                       void* stream) {
+    const int32_t rc = ray_setup_check(k_inv, n_k, sdd, n_s, batch, height, width, n_samples);
+    if (rc != NDRR_OK) return rc;
+    if (src == nullptr || tgt == nullptr || step == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "src, tgt and step must be non-NULL");
+    const cudaError_t e = ndrr::launch_ray_setup(k_inv, n_k, sdd, n_s, batch, height, width, orthographic != 0, n_samples,
+                                                 src, tgt, step, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "ray set-up launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_ray_setup_bwd_workspace_bytes(int32_t batch, int32_t height, int32_t width, uint64_t* bytes) {
+    if (bytes == nullptr || batch < 1 || height < 1 || width < 1 ||
+        (long long)batch * height * width * 3 >= (1LL << 31))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "bad ray set-up shape");
+    *bytes = ndrr::ray_setup_workspace_bytes(batch, height, width);
+    return ok();
+}
+
+int32_t ndrr_ray_setup_bwd(const float* k_inv, int32_t n_k, const float* sdd, int32_t n_s, int32_t batch,
+                           int32_t height, int32_t width, int32_t orthographic, int32_t n_samples, const float* gsrc,
+                           const float* gtgt, const float* gstep, float* g_k, float* g_sdd, void* workspace,
+                           uint64_t workspace_bytes, void* stream) {
+    const int32_t rc = ray_setup_check(k_inv, n_k, sdd, n_s, batch, height, width, n_samples);
+    if (rc != NDRR_OK) return rc;
+    if (g_k == nullptr || g_sdd == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "g_k and g_sdd must be non-NULL");
+    const uint64_t need = ndrr::ray_setup_workspace_bytes(batch, height, width);
+    if (workspace == nullptr || workspace_bytes < need || misaligned(workspace, 4))
+        return fail(NDRR_ERR_WORKSPACE, "the ray set-up adjoint needs %llu workspace bytes, got %llu",
+                    (unsigned long long)need, (unsigned long long)(workspace ? workspace_bytes : 0));
+    const cudaError_t e = ndrr::launch_ray_setup_bwd(k_inv, n_k, sdd, n_s, batch, height, width, orthographic != 0,
+                                                     n_samples, gsrc, gtgt, gstep, g_k, g_sdd, workspace,
+                                                     reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "ray set-up adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_camera_affine(const float* w2v, const float* rt, int32_t batch, float* M, float* M_lo, void* stream) {
+    if (batch < 1 || batch >= (1 << 27) || w2v == nullptr || rt == nullptr || M == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "w2v, rt and M must be non-NULL and batch in 1 .. 2^27 (got %d)", batch);
+    const cudaError_t e =
+        ndrr::launch_camera_affine(w2v, rt, batch, M, M_lo, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "affine launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_camera_affine_bwd(const float* w2v, const float* gM, int32_t batch, float* g_rt, void* stream) {
+    if (batch < 1 || batch >= (1 << 27) || w2v == nullptr || gM == nullptr || g_rt == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "w2v, gM and g_rt must be non-NULL and batch in 1 .. 2^27 (got %d)", batch);
+    const cudaError_t e = ndrr::launch_camera_affine_bwd(w2v, gM, batch, g_rt, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "affine adjoint launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
 int32_t ndrr_set_kernel_events(void* start, void* stop) {
     if ((start == nullptr) != (stop == nullptr))
         return fail(NDRR_ERR_INVALID_ARGUMENT, "start and stop events are both set or both NULL");

@@ -75,6 +75,14 @@ cudaError_t launch_batched(const ndrr_batch_args& a, bool backward, int sm_count
 cudaError_t device_flags(unsigned* out, bool clear);
 cudaError_t launch_camera_rays(const float* k_inv, int n_k, const float* sdd, int n_s, int B, int height, int width,
                                int orthographic, float* src, float* tgt, cudaStream_t st);
+cudaError_t launch_ray_setup(const float* k_inv, int n_k, const float* sdd, int n_s, int B, int height, int width,
+                             int orthographic, int n_samples, float* src, float* tgt, float* step, cudaStream_t st);
+uint64_t ray_setup_workspace_bytes(int B, int height, int width);
+cudaError_t launch_ray_setup_bwd(const float* k_inv, int n_k, const float* sdd, int n_s, int B, int height, int width,
+                                 int orthographic, int n_samples, const float* gsrc, const float* gtgt,
+                                 const float* gstep, float* g_k, float* g_s, void* workspace, cudaStream_t st);
+cudaError_t launch_camera_affine(const float* w2v, const float* rt, int B, float* M, float* M_lo, cudaStream_t st);
+cudaError_t launch_camera_affine_bwd(const float* w2v, const float* gM, int B, float* g_rt, cudaStream_t st);
 cudaError_t launch_hu_to_mu(const void* hu, int dtype, long long n, float mu_water, float dmu, float hu_bone,
                             void* mu, cudaStream_t st);
 cudaError_t launch_occupancy(const void* vol, int vol_dtype, int D, int H, int W, int cell, int max_dist,

@@ -728,9 +728,12 @@ def _ex_setup_context(ctx, inputs, output):
      margin, windows_ahead, slab_mib) = inputs
     ctx.save_for_backward(vol, quad, lab, M.contiguous(), M_lo, src, tgt, step, occ_grid, proposal, output[1])
     ctx.args = (n_samples, n_classes, width, occ_cell, mode, margin, slab_mib)
+    ctx.set_materialize_grads(False)  # the windows output has no gradient: no zeros of its size
 
 
 def _ex_backward(ctx, go, _gwin):
+    if go is None:
+        return (None,) * 18
     vol, quad, lab, M, M_lo, src, tgt, step, occ_grid, proposal, windows = ctx.saved_tensors
     n_samples, n_classes, width, occ_cell, mode, margin, slab_mib = ctx.args
     need_gvol = ctx.needs_input_grad[0]

@@ -312,9 +312,12 @@ def _ncc_patch_setup(ctx, inputs, output):
     x1, x2, p, _ = inputs
     ctx.save_for_backward(x1, x2, output[1])
     ctx.p = p
+    ctx.set_materialize_grads(False)
 
 
 def _ncc_patch_backward(ctx, g_score, _g_maps):
+    if g_score is None:
+        return None, None, None, None
     x1, x2, maps = ctx.saved_tensors
     need1, need2 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
     g1, g2 = _ncc_patch_bwd_op(g_score, x1, x2, maps.contiguous(), ctx.p, need1, need2)

@@ -13,6 +13,7 @@ falling back to a CPU path.
 
 from __future__ import annotations
 
+import ctypes
 import weakref
 
 import torch
@@ -118,6 +119,164 @@ def _camera_rays(k_inv, sdd, height, width, orthographic, device, dtype) -> tupl
     return _make_src(orthographic, tgt, sdd), tgt
 
 
+# ------------------------------------------------------------- ray set-up
+# Rays and sample spacing of a call in one launch, and their adjoint to K^-1
+# and sdd in two: as tensor expressions a differentiable camera was 40 launches
+# per step, most of the host time of a small calibration step.
+def _ray_setup_takes(k_inv, sdd, height, width, rt_inv) -> bool:
+    """Float32 CUDA cameras and poses of one device, K^-1 [1 or B, 3, 3] and
+    sdd [1 or B] for B poses; other inputs, and traced calls, use
+    `_camera_rays` and tensor operations."""
+    if hasattr(torch, "compiler") and torch.compiler.is_compiling():
+        return False
+    if not (rt_inv.dtype == k_inv.dtype == sdd.dtype == torch.float32):
+        return False
+    if not (rt_inv.is_cuda and rt_inv.device == k_inv.device == sdd.device):
+        return False
+    if k_inv.dim() != 3 or tuple(k_inv.shape[1:]) != (3, 3) or sdd.dim() != 1 or rt_inv.dim() != 3:
+        return False
+    B = max(rt_inv.shape[0], k_inv.shape[0], sdd.shape[0])
+    return (min(rt_inv.shape[0], height, width) >= 1 and k_inv.shape[0] in (1, B) and sdd.shape[0] in (1, B)
+            and B <= 65535 and 3 * B * height * width < 2**31)
+
+
+def _ray_setup(k_inv, sdd, batch, height, width, n_samples, orthographic):
+    """(src, tgt, step) of `batch` poses, expanded and contiguous."""
+    k, s = k_inv.detach().contiguous(), sdd.detach().contiguous()
+    N = height * width
+    tgt = torch.empty(batch, N, 3, device=k.device)
+    src = torch.empty(batch, N if orthographic else 1, 3, device=k.device)
+    step = torch.empty(batch, N, device=k.device)
+    _ffi.check(
+        _ffi.load().ndrr_ray_setup(k.data_ptr(), k.shape[0], s.data_ptr(), s.shape[0], batch, height, width,
+                                   int(orthographic), n_samples, src.data_ptr(), tgt.data_ptr(), step.data_ptr(),
+                                   torch.cuda.current_stream(k.device).cuda_stream),
+        "ndrr_ray_setup",
+    )
+    return src, tgt, step
+
+
+@torch.library.custom_op("nanodrr_gb300::ray_setup", mutates_args=())
+def _ray_setup_op(k_inv: torch.Tensor, sdd: torch.Tensor, batch: int, height: int, width: int, n_samples: int,
+                  orthographic: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    return _ray_setup(k_inv, sdd, batch, height, width, n_samples, orthographic)
+
+
+@_ray_setup_op.register_fake
+def _(k_inv, sdd, batch, height, width, n_samples, orthographic):
+    N = height * width
+    return (k_inv.new_empty(batch, N if orthographic else 1, 3), k_inv.new_empty(batch, N, 3),
+            k_inv.new_empty(batch, N))
+
+
+@torch.library.custom_op("nanodrr_gb300::ray_setup_bwd", mutates_args=())
+def _ray_setup_bwd_op(gsrc: torch.Tensor | None, gtgt: torch.Tensor | None, gstep: torch.Tensor | None,
+                      k_inv: torch.Tensor, sdd: torch.Tensor, batch: int, height: int, width: int, n_samples: int,
+                      orthographic: bool) -> tuple[torch.Tensor, torch.Tensor]:
+    k, s = k_inv.contiguous(), sdd.contiguous()
+    grads = [None if g is None else g.float().contiguous() for g in (gsrc if orthographic else None, gtgt, gstep)]
+    g_k = torch.empty(batch, 3, 3, device=k.device)
+    g_s = torch.empty(batch, device=k.device)
+    lib = _ffi.load()
+    nb = ctypes.c_uint64(0)
+    _ffi.check(lib.ndrr_ray_setup_bwd_workspace_bytes(batch, height, width, ctypes.byref(nb)), "workspace query")
+    ws = torch.empty(int(nb.value), device=k.device, dtype=torch.uint8)
+    _ffi.check(
+        lib.ndrr_ray_setup_bwd(k.data_ptr(), k.shape[0], s.data_ptr(), s.shape[0], batch, height, width,
+                               int(orthographic), n_samples, *(None if g is None else g.data_ptr() for g in grads),
+                               g_k.data_ptr(), g_s.data_ptr(), ws.data_ptr(), ws.numel(),
+                               torch.cuda.current_stream(k.device).cuda_stream),
+        "ndrr_ray_setup_bwd",
+    )
+    if batch > 1:  # one camera shared by the poses: sum over them
+        g_k = g_k.sum(0, keepdim=True) if k.shape[0] == 1 else g_k
+        g_s = g_s.sum(0, keepdim=True) if s.shape[0] == 1 else g_s
+    return g_k, g_s
+
+
+@_ray_setup_bwd_op.register_fake
+def _(gsrc, gtgt, gstep, k_inv, sdd, batch, height, width, n_samples, orthographic):
+    return torch.empty_like(k_inv), torch.empty_like(sdd)
+
+
+def _ray_setup_context(ctx, inputs, output):
+    ctx.save_for_backward(inputs[0], inputs[1])
+    ctx.args = inputs[2:]
+    ctx.set_materialize_grads(False)
+
+
+def _ray_setup_backward(ctx, gsrc, gtgt, gstep):
+    k_inv, sdd = ctx.saved_tensors
+    g_k, g_s = _ray_setup_bwd_op(gsrc, gtgt, gstep, k_inv, sdd, *ctx.args)
+    return (g_k if ctx.needs_input_grad[0] else None, g_s if ctx.needs_input_grad[1] else None, *[None] * 5)
+
+
+torch.library.register_autograd("nanodrr_gb300::ray_setup", _ray_setup_backward, setup_context=_ray_setup_context)
+
+
+# --------------------------------------------------------- camera -> voxel
+def _affine_takes(w2v: torch.Tensor, rt_inv: torch.Tensor) -> bool:
+    """Float32 affine and poses on one CUDA device, the affine without a
+    gradient, outside tracing; others use `_affine_product`."""
+    return (not (hasattr(torch, "compiler") and torch.compiler.is_compiling())
+            and rt_inv.is_cuda and w2v.device == rt_inv.device and w2v.dtype == rt_inv.dtype == torch.float32
+            and tuple(w2v.shape) == (4, 4) and rt_inv.dim() == 3 and rt_inv.shape[0] >= 1
+            and tuple(rt_inv.shape[1:]) == (4, 4) and not w2v.requires_grad)
+
+
+def _camera_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, low: bool) -> tuple[torch.Tensor, torch.Tensor]:
+    w, rt = w2v.detach().contiguous(), rt_inv.detach().contiguous()
+    B = rt.shape[0]
+    M = torch.empty(B, 3, 4, device=rt.device)
+    M_lo = torch.empty(B, 3, 4, device=rt.device) if low else M.new_empty(0)
+    _ffi.check(_ffi.load().ndrr_camera_affine(w.data_ptr(), rt.data_ptr(), B, M.data_ptr(),
+                                              M_lo.data_ptr() if low else None,
+                                              torch.cuda.current_stream(rt.device).cuda_stream), "ndrr_camera_affine")
+    return M, M_lo
+
+
+@torch.library.custom_op("nanodrr_gb300::camera_affine", mutates_args=())
+def _camera_affine_op(w2v: torch.Tensor, rt_inv: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """M = (world_to_voxel @ rt_inv)[:, :3] in float32 and its low parts."""
+    return _camera_affine(w2v, rt_inv, True)
+
+
+@_camera_affine_op.register_fake
+def _(w2v, rt_inv):
+    return rt_inv.new_empty(rt_inv.shape[0], 3, 4), rt_inv.new_empty(rt_inv.shape[0], 3, 4)
+
+
+@torch.library.custom_op("nanodrr_gb300::camera_affine_bwd", mutates_args=())
+def _camera_affine_bwd_op(gM: torch.Tensor, w2v: torch.Tensor) -> torch.Tensor:
+    g, w = gM.contiguous(), w2v.contiguous()
+    out = torch.empty(g.shape[0], 4, 4, device=g.device)
+    _ffi.check(_ffi.load().ndrr_camera_affine_bwd(w.data_ptr(), g.data_ptr(), g.shape[0], out.data_ptr(),
+                                                  torch.cuda.current_stream(g.device).cuda_stream),
+               "ndrr_camera_affine_bwd")
+    return out
+
+
+@_camera_affine_bwd_op.register_fake
+def _(gM, w2v):
+    return gM.new_empty(gM.shape[0], 4, 4)
+
+
+def _camera_affine_context(ctx, inputs, output):
+    ctx.save_for_backward(inputs[0])
+    ctx.set_materialize_grads(False)
+
+
+def _camera_affine_backward(ctx, gM, _g_lo):
+    # M_lo is a rounding correction of M, not differentiated
+    if gM is None:
+        return None, None
+    return None, _camera_affine_bwd_op(gM, ctx.saved_tensors[0])
+
+
+torch.library.register_autograd("nanodrr_gb300::camera_affine", _camera_affine_backward,
+                                setup_context=_camera_affine_context)
+
+
 def _affine_product(A3: torch.Tensor, rt: torch.Tensor) -> torch.Tensor:
     """(A @ rt)[:, :3, :] for A3 = A[:3] ([3, 4]) and rt [B, 4, 4], written as a
     broadcast sum (camera -> voxel affine of the reference, backends.py:96)."""
@@ -128,9 +287,14 @@ def _call_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, grad: bool) -> torch.T
     """M = (world_to_voxel @ rt_inv)[:, :3] in float32 (`_affine_product`),
     from the affine cache when no gradient is recorded and nothing is traced
     or captured into a CUDA graph (a graph must read rt_inv on every replay)."""
+    def product():
+        if not grad and _affine_takes(w2v, rt_inv):
+            return _camera_affine(w2v, rt_inv, False)[0]
+        return _affine_product(w2v.float()[:3], rt_inv.float())
+
     if (grad or (hasattr(torch, "compiler") and torch.compiler.is_compiling())
             or rt_inv.device.type != "cuda" or torch.cuda.is_current_stream_capturing()):
-        return _affine_product(w2v.float()[:3], rt_inv.float())
+        return product()
     stream = torch.cuda.current_stream(rt_inv.device)
     key = (id(w2v), id(rt_inv))
     hit = _M_CACHE.get(key)
@@ -140,7 +304,7 @@ def _call_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, grad: bool) -> torch.T
             if stream != made_on:  # keep the allocator from reusing it under this stream's kernels
                 M.record_stream(stream)
             return M
-    M = _affine_product(w2v.float()[:3], rt_inv.float())
+    M = product()
     for k in [k for k, v in _M_CACHE.items() if v[0]() is None or v[2]() is None]:
         del _M_CACHE[k]  # entries whose tensors are gone
     while len(_M_CACHE) >= _M_CACHE_SIZE:
@@ -184,12 +348,19 @@ def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) 
     # the float64 affine of the same inputs. The forward reads float32 M only,
     # so a call without a gradient skips the float64 product.
     grad = torch.is_grad_enabled() and any(t.requires_grad for t in (vol, rt_inv, src, tgt, step_size))
-    M = _call_affine(subject.world_to_voxel, rt_inv, grad)
-    if grad:
+    if grad and _affine_takes(subject.world_to_voxel, rt_inv):
+        if rt_inv.requires_grad:
+            M, M_lo = _camera_affine_op(subject.world_to_voxel, rt_inv)
+            M_lo = M_lo.detach()
+        else:
+            M, M_lo = _camera_affine(subject.world_to_voxel, rt_inv, True)
+    elif not grad:
+        M = _call_affine(subject.world_to_voxel, rt_inv, grad)
+        M_lo = M.new_empty(0)
+    else:
+        M = _call_affine(subject.world_to_voxel, rt_inv, grad)
         M64 = _affine_product(subject.world_to_voxel.detach().double()[:3], rt_inv.detach().double())
         M_lo = (M64 - M.detach().double()).float()
-    else:
-        M_lo = M.new_empty(0)
     B = max(M.shape[0], tgt.shape[0])
     if M.shape[0] != B:
         M = M.expand(B, -1, -1)
@@ -305,6 +476,12 @@ def render(
         rays = _cached_rays(k_inv, sdd, height, width, n_samples, orthographic, rt_inv)
         if rays is not None:
             return render_cuda(subject, rt_inv, *rays, n_samples, height, width)
+        if _ray_setup_takes(k_inv, sdd, height, width, rt_inv):
+            B = max(rt_inv.shape[0], k_inv.shape[0], sdd.shape[0])
+            args = (k_inv, sdd, B, height, width, n_samples, bool(orthographic))
+            live = torch.is_grad_enabled() and (k_inv.requires_grad or sdd.requires_grad)
+            rays = (_ray_setup_op if live else _ray_setup)(*args)
+            return render_cuda(subject, rt_inv, *rays, n_samples, height, width)
     if tgt is None and src is None:
         src, tgt = _camera_rays(k_inv, sdd, height, width, orthographic, device, dtype)
     if tgt is None:
@@ -339,10 +516,13 @@ def _cached_rays(k_inv, sdd, height, width, n_samples, orthographic, rt_inv):
                 for t in rays:
                     t.record_stream(stream)
             return rays
-    src, tgt = _camera_rays(k_inv, sdd, height, width, orthographic, device, dtype)
-    step = (tgt - src).norm(dim=-1) / float(n_samples - 1)
-    rays = (src.expand(B, -1, -1).float().contiguous(), tgt.expand(B, -1, -1).float().contiguous(),
-            step.expand(B, -1).float().contiguous())
+    if _ray_setup_takes(k_inv, sdd, height, width, rt_inv):
+        rays = _ray_setup(k_inv, sdd, B, height, width, n_samples, bool(orthographic))
+    else:
+        src, tgt = _camera_rays(k_inv, sdd, height, width, orthographic, device, dtype)
+        step = (tgt - src).norm(dim=-1) / float(n_samples - 1)
+        rays = (src.expand(B, -1, -1).float().contiguous(), tgt.expand(B, -1, -1).float().contiguous(),
+                step.expand(B, -1).float().contiguous())
     for k in [k for k, v in _RAY_CACHE.items() if v[0]() is None or v[2]() is None]:
         del _RAY_CACHE[k]  # entries whose camera tensors are gone
     while len(_RAY_CACHE) >= _RAY_CACHE_SIZE:
