@@ -950,13 +950,16 @@ __device__ __forceinline__ void bwd_body(const MarchParams& p, const int tile, c
 }
 
 // Register budget of the adjoint: 128 (one CTA of 512 threads per SM), but
-// 72 for the one-channel pose-only adjoint of an f32 quad volume without an
-// in-kernel skip, where occupancy pays: 0.70 ms, against 0.78 at 56 and 0.73
-// at 80 (512 x 512 x 400, 16 poses x 200^2, 500 samples, kernel alone).
+// 72 for the pose-only adjoints of a quad layout where occupancy pays: one
+// channel f32 without an in-kernel skip 0.70 ms, against 0.78 at 56 and 0.73
+// at 80 (512 x 512 x 400, 16 poses x 200^2, 500 samples, kernel alone); 8
+// label channels bf16 3.41 ms, against 3.71 uncapped and 3.52 at 80 (32 poses x
+// 256^2, 800 samples).
 template <typename VT, bool MULTI, bool GVOL, bool GCAM, int SKIP, int QUAD>
 struct BwdRegs {
-    static constexpr int value =
-        (!MULTI && !GVOL && !GCAM && SKIP == 0 && QUAD == kLayoutQuad && std::is_same<VT, float>::value) ? 72 : 128;
+    static constexpr bool pose_quad = !GVOL && !GCAM && QUAD != kLayoutVolume;
+    static constexpr bool one_f32 = !MULTI && SKIP == 0 && std::is_same<VT, float>::value;
+    static constexpr int value = pose_quad && (MULTI || one_f32) ? 72 : 128;
 };
 
 template <typename VT, bool MULTI, bool GVOL, bool GCAM, int SKIP, int QUAD>

@@ -29,18 +29,14 @@ __device__ __forceinline__ bool grid_interval(const OccGrid& g, const Ray& r, fl
     return t0 <= t1;
 }
 
-// Parameter at which the ray, currently inside the voxel box [lo, hi) on every
-// axis, leaves it (the nearest exit face in the direction of travel).
-__device__ __forceinline__ float box_exit(const Ray& r, float t, float lox, float hix, float loy, float hiy,
-                                          float loz, float hiz) {
-    float te = INFINITY;
-    if (r.dx > 0.f) te = fminf(te, (hix - r.p0x) / r.dx);
-    if (r.dx < 0.f) te = fminf(te, (lox - r.p0x) / r.dx);
-    if (r.dy > 0.f) te = fminf(te, (hiy - r.p0y) / r.dy);
-    if (r.dy < 0.f) te = fminf(te, (loy - r.p0y) / r.dy);
-    if (r.dz > 0.f) te = fminf(te, (hiz - r.p0z) / r.dz);
-    if (r.dz < 0.f) te = fminf(te, (loz - r.p0z) / r.dz);
-    return fmaxf(te, t);
+// Parameter at which the ray, currently inside the cube of voxels from cell
+// corner lo to hi on every axis, leaves it: the nearest exit face in the
+// direction of travel. `inv` holds 1 / d (0 for an axis the ray does not move
+// along), one reciprocal per axis and walk instead of a division per face and
+// step; its rounding (1e-7 of the parameter, under 1e-4 voxel) is inside the
+// step's margin of 1e-3 voxel (windows of 8.4 M rays: 727 -> 559 us).
+__device__ __forceinline__ float axis_exit(float p, float inv, float lo, float hi) {
+    return inv == 0.f ? INFINITY : ((inv > 0.f ? hi : lo) - p) * inv;
 }
 
 // March the distance field from ta toward tb (tb < ta marches backward).
@@ -66,6 +62,8 @@ __device__ __forceinline__ int first_occupied(const OccGrid& g, Ray r, float ta,
     const float c = (float)g.cell, inv_c = 1.0f / c;
     const float dmax = fmaxf(fmaxf(fabsf(r.dx), fabsf(r.dy)), fabsf(r.dz));
     const float eps = dmax > 0.f ? 1e-3f / dmax : 1e30f;  // a thousandth of a voxel
+    const float ix = r.dx != 0.f ? 1.0f / r.dx : 0.f, iy = r.dy != 0.f ? 1.0f / r.dy : 0.f,
+                iz = r.dz != 0.f ? 1.0f / r.dz : 0.f;
     for (int it = 0; it < max_steps; ++it) {
         if (t > tend) return 0;
         const float px = fmaf(t, r.dx, r.p0x), py = fmaf(t, r.dy, r.p0y), pz = fmaf(t, r.dz, r.p0z);
@@ -78,10 +76,10 @@ __device__ __forceinline__ int first_occupied(const OccGrid& g, Ray r, float ta,
             return 1;
         }
         // Empty cube of cells [c - d + 1, c + d - 1] -> voxels [(c - d) cell, (c + d - 1) cell).
-        const float lox = (float)(cx - d) * c, hix = (float)(cx + d - 1) * c;
-        const float loy = (float)(cy - d) * c, hiy = (float)(cy + d - 1) * c;
-        const float loz = (float)(cz - d) * c, hiz = (float)(cz + d - 1) * c;
-        t = box_exit(r, t, lox, hix, loy, hiy, loz, hiz) + eps;
+        const float te = fminf(fminf(axis_exit(r.p0x, ix, (float)(cx - d) * c, (float)(cx + d - 1) * c),
+                                     axis_exit(r.p0y, iy, (float)(cy - d) * c, (float)(cy + d - 1) * c)),
+                               axis_exit(r.p0z, iz, (float)(cz - d) * c, (float)(cz + d - 1) * c));
+        t = fmaxf(te, t) + eps;
     }
     return -1;
 }
