@@ -1,0 +1,28 @@
+"""When an adjoint may be called without its operator.
+
+The library's adjoints are registered operators, so that traced and transformed
+graphs see them; an operator call costs 100 to 150 us of host time on the Arm
+host, most of a small step. A plain eager backward needs none of that and calls
+the function behind the operator.
+"""
+
+from __future__ import annotations
+
+import torch
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+_dispatch_modes = getattr(torch._C, "_len_torch_dispatch_stack", None)
+_functorch = getattr(torch._C, "_functorch", None)
+_interpreters = getattr(_functorch, "peek_interpreter_stack", None)
+
+
+def plain_eager(*tensors) -> bool:
+    """Ordinary tensors (no fake, functional or other subclass), no gradient
+    recorded (a double backward must meet the operator, which refuses it), no
+    compiler, dispatch mode or function transform active. Where this torch
+    cannot tell, the operator is called."""
+    if _dispatch_modes is None or _interpreters is None or torch.is_grad_enabled():
+        return False
+    if any(t is not None and type(t) not in _PLAIN for t in tensors):
+        return False
+    return not torch.compiler.is_compiling() and _dispatch_modes() == 0 and _interpreters() is None

@@ -11,6 +11,8 @@ import ctypes
 import threading
 from pathlib import Path
 
+import torch
+
 from . import _build
 
 # ndrr_status
@@ -234,6 +236,8 @@ def library_path() -> Path:
 def load(build_if_missing: bool = True) -> ctypes.CDLL:
     """Load (building first if needed) the shared library and bind signatures."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -267,3 +271,14 @@ def check(rc: int, what: str) -> None:
     if rc in (NDRR_ERR_INVALID_ARGUMENT, NDRR_ERR_LIMIT, NDRR_ERR_DTYPE):
         raise ValueError(text)
     raise NdrrError(text)
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_handle(device: torch.device) -> int:
+    """The cudaStream_t of the device's current stream (without building the
+    stream object where torch allows it: a few microseconds per launch)."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream

@@ -220,14 +220,14 @@ class BatchedRenderer:
     def forward(self) -> None:
         a = self._args(False)
         lib = _ffi.load()
-        _ffi.check(lib.ndrr_batched_fwd(ctypes.byref(a), torch.cuda.current_stream(self.device).cuda_stream),
+        _ffi.check(lib.ndrr_batched_fwd(ctypes.byref(a), _ffi.stream_handle(self.device)),
                    "ndrr_batched_fwd")
 
     def backward(self) -> None:
         """Pose adjoint of `go_flat` into gM (per request [3, 4])."""
         a = self._args(True)
         lib = _ffi.load()
-        _ffi.check(lib.ndrr_batched_bwd(ctypes.byref(a), torch.cuda.current_stream(self.device).cuda_stream),
+        _ffi.check(lib.ndrr_batched_bwd(ctypes.byref(a), _ffi.stream_handle(self.device)),
                    "ndrr_batched_bwd")
 
     def output(self, i: int) -> torch.Tensor:

@@ -40,7 +40,7 @@ FEATURES = 64
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return _ffi.stream_handle(device)
 
 
 def _root(t: torch.Tensor) -> torch.Tensor:

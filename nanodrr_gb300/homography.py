@@ -17,6 +17,7 @@ import ctypes
 import torch
 
 from . import _ffi
+from ._eager import plain_eager
 from .geometry import mm_small
 
 
@@ -35,7 +36,7 @@ def _inv3(A: torch.Tensor) -> torch.Tensor:
 
 
 def _stream(dev) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    return _ffi.stream_handle(dev)
 
 
 def _check(img: torch.Tensor, hom: torch.Tensor):
@@ -135,9 +136,8 @@ def _(img, k_old, k_new):
     return torch.empty(img.shape, device=img.device, dtype=img.dtype), img.new_empty(img.shape[0], 3, 3)
 
 
-@torch.library.custom_op("nanodrr_gb300::resample_bwd", mutates_args=())
-def _resample_bwd_op(go: torch.Tensor, img: torch.Tensor, hom: torch.Tensor, k_old: torch.Tensor, k_new: torch.Tensor,
-                     need_gimg: bool, need_gk: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+def _resample_bwd(go: torch.Tensor, img: torch.Tensor, hom: torch.Tensor, k_old: torch.Tensor, k_new: torch.Tensor,
+                  need_gimg: bool, need_gk: bool) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     img = img.contiguous()
     go = go.float().contiguous()
     a, b = k_old.float().contiguous(), k_new.float().contiguous()
@@ -158,6 +158,9 @@ def _resample_bwd_op(go: torch.Tensor, img: torch.Tensor, hom: torch.Tensor, k_o
     return gimg, g_old, g_new
 
 
+_resample_bwd_op = torch.library.custom_op("nanodrr_gb300::resample_bwd", mutates_args=())(_resample_bwd)
+
+
 @_resample_bwd_op.register_fake
 def _(go, img, hom, k_old, k_new, need_gimg, need_gk):
     f = lambda t, on: t.new_empty(t.shape if on else (0,) + t.shape[1:], dtype=torch.float32)  # noqa: E731
@@ -172,7 +175,8 @@ def _resample_setup(ctx, inputs, output):
 def _resample_backward(ctx, go, _g_hom):
     img, k_old, k_new, hom = ctx.saved_tensors
     need_gimg, need_old, need_new = ctx.needs_input_grad
-    gimg, g_old, g_new = _resample_bwd_op(go, img, hom, k_old, k_new, need_gimg, need_old or need_new)
+    bwd = _resample_bwd if plain_eager(go, img, hom, k_old, k_new) else _resample_bwd_op
+    gimg, g_old, g_new = bwd(go, img, hom, k_old, k_new, need_gimg, need_old or need_new)
     return (gimg if need_gimg else None, g_old.to(k_old.dtype) if need_old else None,
             g_new.to(k_new.dtype) if need_new else None)
 

@@ -24,6 +24,7 @@ import ctypes
 import torch
 
 from . import _ffi
+from ._eager import plain_eager
 
 _TORCH_TO_NDRR = {
     torch.float32: _ffi.NDRR_F32,
@@ -46,8 +47,7 @@ def ndrr_dtype(t: torch.Tensor) -> int:
         raise ValueError(f"unsupported dtype {t.dtype}") from None
 
 
-def _stream_handle(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+_stream_handle = _ffi.stream_handle
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -377,6 +377,30 @@ def raymarch_forward(
     return out, total
 
 
+def march_direct(vol, quad, lab, M, src, tgt, step, n_samples, n_classes, width, skip=None) -> torch.Tensor:
+    """[B, C, N] forward of a render call that records no gradient:
+    `raymarch_forward` for tensors the caller has made contiguous (float32 but
+    for the volume and labels), `quad` a quad copy or None."""
+    _check_inputs(vol, lab, M, src, tgt, step, n_samples, n_classes)
+    windows = None
+    if _windows_route(skip):
+        windows = skip_windows(vol, M, src, tgt, step, n_samples, width, skip)
+        skip = None
+    out = torch.empty(tgt.shape[0], n_classes, tgt.shape[1], device=vol.device, dtype=vol.dtype)
+    a = _base_args(vol, lab, M, src, tgt, step, n_samples, n_classes, width)
+    a.out = _ptr(out)
+    a.out_dtype = a.vol_dtype
+    if skip is not None:
+        _apply_skip(a, skip, vol)
+    if windows is not None:
+        a.sample_window = _ptr(windows)
+    if quad is not None:
+        a.vol_quad = quad.data_ptr()
+        a.quad_labels = int(quad_is_labeled(vol, quad))
+    _ffi.check(_ffi.load().ndrr_raymarch_fwd(ctypes.byref(a), _stream_handle(vol.device)), "ndrr_raymarch_fwd")
+    return out
+
+
 def raymarch_backward(
     go: torch.Tensor,
     vol: torch.Tensor,
@@ -521,8 +545,7 @@ def _(vol, lab, M, src, tgt, step, n_samples, n_classes, width):
     return torch.empty(B, n_classes, N, device=vol.device, dtype=vol.dtype)
 
 
-@torch.library.custom_op("nanodrr_gb300::fused_raymarch_bwd", mutates_args=())
-def fused_raymarch_bwd(
+def _bwd(
     go: torch.Tensor,
     vol: torch.Tensor,
     lab: torch.Tensor,
@@ -546,6 +569,9 @@ def fused_raymarch_bwd(
         go, vol, lab, M, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam
     )
     return gvol, gM, gsrc, gtgt, gstep
+
+
+fused_raymarch_bwd = torch.library.custom_op("nanodrr_gb300::fused_raymarch_bwd", mutates_args=())(_bwd)
 
 
 @fused_raymarch_bwd.register_fake
@@ -572,7 +598,8 @@ def _backward(ctx, go):
     vol, lab, M, src, tgt, step = ctx.saved_tensors
     need_gvol = ctx.needs_input_grad[0]
     need_gcam = any(ctx.needs_input_grad[i] for i in (3, 4, 5))
-    gvol, gM, gsrc, gtgt, gstep = fused_raymarch_bwd(
+    bwd = _bwd if plain_eager(go, vol, M, src, tgt, step) else fused_raymarch_bwd
+    gvol, gM, gsrc, gtgt, gstep = bwd(
         go, vol, lab, M, src, tgt, step, ctx.n_samples, ctx.n_classes, ctx.width, need_gvol, need_gcam
     )
     return (
@@ -600,13 +627,14 @@ torch.library.register_autograd("nanodrr_gb300::fused_raymarch", _backward, setu
 # gradients equal the plain march's; the volume gradient is computed over the
 # full box-culled window.
 class _SkipArgs:
-    def __init__(self, grid, cell, packed, mode, margin, shape):
+    def __init__(self, grid, cell, packed, mode, margin, shape, fused=True):
         from .empty_space import OccupancyGrid
 
         self.grid = OccupancyGrid(grid, cell, shape)
         self.packed = packed
         self.mode = mode
         self.margin = margin
+        self.fused = fused
 
 
 def _skip_of(vol, occ_grid, occ_cell, proposal, skip_mode, margin):
@@ -672,8 +700,7 @@ def _(vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, occ_
     return out, torch.empty(shape, device=vol.device, dtype=torch.int32)
 
 
-@torch.library.custom_op("nanodrr_gb300::fused_raymarch_ex_bwd", mutates_args=())
-def fused_raymarch_ex_bwd(
+def _ex_bwd(
     go: torch.Tensor,
     vol: torch.Tensor,
     quad: torch.Tensor,
@@ -711,6 +738,9 @@ def fused_raymarch_ex_bwd(
     )
 
 
+fused_raymarch_ex_bwd = torch.library.custom_op("nanodrr_gb300::fused_raymarch_ex_bwd", mutates_args=())(_ex_bwd)
+
+
 @fused_raymarch_ex_bwd.register_fake
 def _(go, vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam, *rest):
     B, N, _ = tgt.shape
@@ -738,7 +768,8 @@ def _ex_backward(ctx, go, _gwin):
     n_samples, n_classes, width, occ_cell, mode, margin, slab_mib = ctx.args
     need_gvol = ctx.needs_input_grad[0]
     need_gcam = any(ctx.needs_input_grad[i] for i in (5, 6, 7))
-    gvol, gM, gsrc, gtgt, gstep = fused_raymarch_ex_bwd(
+    bwd = _ex_bwd if plain_eager(go, vol, M, src, tgt, step) else fused_raymarch_ex_bwd
+    gvol, gM, gsrc, gtgt, gstep = bwd(
         go, vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam,
         occ_grid, occ_cell, proposal, mode, margin, windows, slab_mib,
     )

@@ -19,6 +19,7 @@ import ctypes
 import torch
 
 from . import _ffi
+from ._eager import plain_eager
 from .geometry import convert, mm_small, transform_point
 from .renderer import build_quad, quad_cache_key, render
 
@@ -93,7 +94,7 @@ def _so3_pose_op(rot: torch.Tensor, xyz: torch.Tensor, rt_inv: torch.Tensor, piv
     pose = torch.empty(B, 4, 4, device=rt_inv.device)
     _ffi.check(_ffi.load().ndrr_pose_so3_fwd(r.data_ptr(), x.data_ptr(), rows, a.data_ptr(), p.data_ptr(),
                                              c.data_ptr(), B, pose.data_ptr(),
-                                             torch.cuda.current_stream(rt_inv.device).cuda_stream),
+                                             _ffi.stream_handle(rt_inv.device)),
                "ndrr_pose_so3_fwd")
     return pose.to(rt_inv.dtype)
 
@@ -103,20 +104,22 @@ def _(rot, xyz, rt_inv, pivot, pivot_inv):
     return rt_inv.new_empty(rt_inv.shape[0], 4, 4)
 
 
-@torch.library.custom_op("nanodrr_gb300::so3_pose_bwd", mutates_args=())
-def _so3_pose_bwd_op(gpose: torch.Tensor, rot: torch.Tensor, xyz: torch.Tensor, rt_inv: torch.Tensor,
-                     pivot: torch.Tensor, pivot_inv: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+def _so3_pose_bwd(gpose: torch.Tensor, rot: torch.Tensor, xyz: torch.Tensor, rt_inv: torch.Tensor,
+                  pivot: torch.Tensor, pivot_inv: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     B, rows, r, x, a, p, c = _pose_inputs(rot, xyz, rt_inv, pivot, pivot_inv)
     g = gpose.float().contiguous()
     g_rot = torch.empty(B, 3, device=rt_inv.device)
     g_xyz = torch.empty(B, 3, device=rt_inv.device)
     _ffi.check(_ffi.load().ndrr_pose_so3_bwd(g.data_ptr(), r.data_ptr(), x.data_ptr(), rows, a.data_ptr(),
                                              p.data_ptr(), c.data_ptr(), B, g_rot.data_ptr(), g_xyz.data_ptr(),
-                                             torch.cuda.current_stream(rt_inv.device).cuda_stream),
+                                             _ffi.stream_handle(rt_inv.device)),
                "ndrr_pose_so3_bwd")
     if rows == 1 and B > 1:  # a broadcast parameter: sum over the poses
         g_rot, g_xyz = g_rot.sum(0, keepdim=True), g_xyz.sum(0, keepdim=True)
     return g_rot, g_xyz
+
+
+_so3_pose_bwd_op = torch.library.custom_op("nanodrr_gb300::so3_pose_bwd", mutates_args=())(_so3_pose_bwd)
 
 
 @_so3_pose_bwd_op.register_fake
@@ -133,7 +136,8 @@ def _so3_pose_backward(ctx, gpose):
     if any(ctx.needs_input_grad[2:]):
         raise RuntimeError("so3_pose differentiates the rotation and translation only; rt_inv, pivot and "
                            "pivot_inv are fixed buffers")
-    g_rot, g_xyz = _so3_pose_bwd_op(gpose, rot, xyz, rt_inv, pivot, pivot_inv)
+    bwd = _so3_pose_bwd if plain_eager(gpose, rot, xyz, rt_inv, pivot, pivot_inv) else _so3_pose_bwd_op
+    g_rot, g_xyz = bwd(gpose, rot, xyz, rt_inv, pivot, pivot_inv)
     return g_rot.to(rot.dtype), g_xyz.to(xyz.dtype), None, None, None
 
 
@@ -190,7 +194,7 @@ def _ncc_op(x1: torch.Tensor, x2: torch.Tensor, eps: float) -> tuple[torch.Tenso
     _ffi.check(lib.ndrr_ncc_workspace_bytes(B, C, H * W, ctypes.byref(nb)), "ndrr_ncc_workspace_bytes")
     ws = torch.empty(max(int(nb.value), 16), device=x1.device, dtype=torch.uint8)
     _ffi.check(lib.ndrr_ncc_fwd(a.data_ptr(), b.data_ptr(), B, C, H * W, eps, score.data_ptr(), stats.data_ptr(),
-                                ws.data_ptr(), ws.numel(), torch.cuda.current_stream(x1.device).cuda_stream),
+                                ws.data_ptr(), ws.numel(), _ffi.stream_handle(x1.device)),
                "ndrr_ncc_fwd")
     return score.to(x1.dtype), stats
 
@@ -201,9 +205,8 @@ def _(x1, x2, eps):
     return x1.new_empty(B), x1.new_empty(B, C, 8, dtype=torch.float32)
 
 
-@torch.library.custom_op("nanodrr_gb300::ncc_bwd", mutates_args=())
-def _ncc_bwd_op(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, stats: torch.Tensor, need1: bool,
-                need2: bool) -> tuple[torch.Tensor, torch.Tensor]:
+def _ncc_bwd(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, stats: torch.Tensor, need1: bool,
+             need2: bool) -> tuple[torch.Tensor, torch.Tensor]:
     B, C, H, W = x1.shape
     a, b = x1.float().contiguous(), x2.float().contiguous()
     g1 = torch.empty_like(a) if need1 else a.new_empty(0)
@@ -211,9 +214,12 @@ def _ncc_bwd_op(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, stats: tor
     lib = _ffi.load()
     _ffi.check(lib.ndrr_ncc_bwd(go.float().contiguous().data_ptr(), a.data_ptr(), b.data_ptr(),
                                 stats.contiguous().data_ptr(), B, C, H * W, g1.data_ptr() if need1 else None,
-                                g2.data_ptr() if need2 else None, torch.cuda.current_stream(x1.device).cuda_stream),
+                                g2.data_ptr() if need2 else None, _ffi.stream_handle(x1.device)),
                "ndrr_ncc_bwd")
     return g1, g2
+
+
+_ncc_bwd_op = torch.library.custom_op("nanodrr_gb300::ncc_bwd", mutates_args=())(_ncc_bwd)
 
 
 @_ncc_bwd_op.register_fake
@@ -230,7 +236,8 @@ def _ncc_setup(ctx, inputs, output):
 def _ncc_backward(ctx, g_score, _g_stats):
     x1, x2, stats = ctx.saved_tensors
     need1, need2 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-    g1, g2 = _ncc_bwd_op(g_score, x1, x2, stats, need1, need2)
+    bwd = _ncc_bwd if plain_eager(g_score, x1, x2, stats) else _ncc_bwd_op
+    g1, g2 = bwd(g_score, x1, x2, stats, need1, need2)
     return (g1.to(x1.dtype) if need1 else None, g2.to(x2.dtype) if need2 else None, None)
 
 
@@ -277,7 +284,7 @@ def _ncc_patch_op(x1: torch.Tensor, x2: torch.Tensor, p: int, eps: float) -> tup
     ws = torch.empty(int(nb.value), device=x1.device, dtype=torch.uint8)
     _ffi.check(lib.ndrr_ncc_patch_fwd(a.data_ptr(), b.data_ptr(), B, C, H, W, p, eps, score.data_ptr(),
                                       maps.data_ptr(), ws.data_ptr(), ws.numel(),
-                                      torch.cuda.current_stream(x1.device).cuda_stream), "ndrr_ncc_patch_fwd")
+                                      _ffi.stream_handle(x1.device)), "ndrr_ncc_patch_fwd")
     return score.to(x1.dtype), maps
 
 
@@ -287,9 +294,8 @@ def _(x1, x2, p, eps):
     return x1.new_empty(B), x1.new_empty(B, C, 5, H - p + 1, W - p + 1, dtype=torch.float64)
 
 
-@torch.library.custom_op("nanodrr_gb300::ncc_patch_bwd", mutates_args=())
-def _ncc_patch_bwd_op(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, maps: torch.Tensor, p: int, need1: bool,
-                      need2: bool) -> tuple[torch.Tensor, torch.Tensor]:
+def _ncc_patch_bwd(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, maps: torch.Tensor, p: int, need1: bool,
+                   need2: bool) -> tuple[torch.Tensor, torch.Tensor]:
     B, C, H, W = x1.shape
     a, b = x1.float().contiguous(), x2.float().contiguous()
     g1 = torch.empty_like(a) if need1 else a.new_empty(0)
@@ -297,8 +303,11 @@ def _ncc_patch_bwd_op(go: torch.Tensor, x1: torch.Tensor, x2: torch.Tensor, maps
     g = go.float().contiguous()
     _ffi.check(_ffi.load().ndrr_ncc_patch_bwd(g.data_ptr(), a.data_ptr(), b.data_ptr(), maps.data_ptr(), B, C, H, W, p,
                                               g1.data_ptr() if need1 else None, g2.data_ptr() if need2 else None,
-                                              torch.cuda.current_stream(x1.device).cuda_stream), "ndrr_ncc_patch_bwd")
+                                              _ffi.stream_handle(x1.device)), "ndrr_ncc_patch_bwd")
     return g1, g2
+
+
+_ncc_patch_bwd_op = torch.library.custom_op("nanodrr_gb300::ncc_patch_bwd", mutates_args=())(_ncc_patch_bwd)
 
 
 @_ncc_patch_bwd_op.register_fake
@@ -320,7 +329,8 @@ def _ncc_patch_backward(ctx, g_score, _g_maps):
         return None, None, None, None
     x1, x2, maps = ctx.saved_tensors
     need1, need2 = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-    g1, g2 = _ncc_patch_bwd_op(g_score, x1, x2, maps.contiguous(), ctx.p, need1, need2)
+    bwd = _ncc_patch_bwd if plain_eager(g_score, x1, x2, maps) else _ncc_patch_bwd_op
+    g1, g2 = bwd(g_score, x1, x2, maps.contiguous(), ctx.p, need1, need2)
     return (g1.to(x1.dtype) if need1 else None, g2.to(x2.dtype) if need2 else None, None, None)
 
 

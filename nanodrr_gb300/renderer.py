@@ -19,9 +19,11 @@ import weakref
 import torch
 
 from . import _ffi
+from ._eager import plain_eager
 from .raymarch import (
+    _SkipArgs,
     fused_raymarch_ex,
-    fused_raymarch_ex_forward,
+    march_direct,
     quad_volume,
     quad_volume_labeled,
 )
@@ -48,8 +50,11 @@ _M_CACHE_SIZE = 4
 def fused_supported(subject: Subject, B: int, n_pixels: int) -> bool:
     """Limits of the CUDA kernels: one volume, int32 voxel and ray indexing
     (reference backends.py:66-69)."""
-    N = B * n_pixels
-    return subject.image.shape[0] == 1 and max(subject.image.numel(), subject.n_classes * N, 3 * N) < 2**31
+    return _within_limits(subject.image, subject.n_classes, B * n_pixels)
+
+
+def _within_limits(img: torch.Tensor, n_classes: int, n_rays: int) -> bool:
+    return img.shape[0] == 1 and max(img.numel(), n_classes * n_rays, 3 * n_rays) < 2**31
 
 
 def _make_tgt(k_inv, sdd, height, width, device, dtype) -> torch.Tensor:
@@ -111,7 +116,7 @@ def _camera_rays(k_inv, sdd, height, width, orthographic, device, dtype) -> tupl
             lib = _ffi.load()
             _ffi.check(
                 lib.ndrr_camera_rays(k.data_ptr(), n_k, s.data_ptr(), n_s, B, height, width, int(bool(orthographic)),
-                                     src.data_ptr(), tgt.data_ptr(), torch.cuda.current_stream(k.device).cuda_stream),
+                                     src.data_ptr(), tgt.data_ptr(), _ffi.stream_handle(k.device)),
                 "ndrr_camera_rays",
             )
             return src, tgt
@@ -150,7 +155,7 @@ def _ray_setup(k_inv, sdd, batch, height, width, n_samples, orthographic):
     _ffi.check(
         _ffi.load().ndrr_ray_setup(k.data_ptr(), k.shape[0], s.data_ptr(), s.shape[0], batch, height, width,
                                    int(orthographic), n_samples, src.data_ptr(), tgt.data_ptr(), step.data_ptr(),
-                                   torch.cuda.current_stream(k.device).cuda_stream),
+                                   _ffi.stream_handle(k.device)),
         "ndrr_ray_setup",
     )
     return src, tgt, step
@@ -169,10 +174,9 @@ def _(k_inv, sdd, batch, height, width, n_samples, orthographic):
             k_inv.new_empty(batch, N))
 
 
-@torch.library.custom_op("nanodrr_gb300::ray_setup_bwd", mutates_args=())
-def _ray_setup_bwd_op(gsrc: torch.Tensor | None, gtgt: torch.Tensor | None, gstep: torch.Tensor | None,
-                      k_inv: torch.Tensor, sdd: torch.Tensor, batch: int, height: int, width: int, n_samples: int,
-                      orthographic: bool) -> tuple[torch.Tensor, torch.Tensor]:
+def _ray_setup_bwd(gsrc: torch.Tensor | None, gtgt: torch.Tensor | None, gstep: torch.Tensor | None,
+                   k_inv: torch.Tensor, sdd: torch.Tensor, batch: int, height: int, width: int, n_samples: int,
+                   orthographic: bool) -> tuple[torch.Tensor, torch.Tensor]:
     k, s = k_inv.contiguous(), sdd.contiguous()
     grads = [None if g is None else g.float().contiguous() for g in (gsrc if orthographic else None, gtgt, gstep)]
     g_k = torch.empty(batch, 3, 3, device=k.device)
@@ -185,13 +189,16 @@ def _ray_setup_bwd_op(gsrc: torch.Tensor | None, gtgt: torch.Tensor | None, gste
         lib.ndrr_ray_setup_bwd(k.data_ptr(), k.shape[0], s.data_ptr(), s.shape[0], batch, height, width,
                                int(orthographic), n_samples, *(None if g is None else g.data_ptr() for g in grads),
                                g_k.data_ptr(), g_s.data_ptr(), ws.data_ptr(), ws.numel(),
-                               torch.cuda.current_stream(k.device).cuda_stream),
+                               _ffi.stream_handle(k.device)),
         "ndrr_ray_setup_bwd",
     )
     if batch > 1:  # one camera shared by the poses: sum over them
         g_k = g_k.sum(0, keepdim=True) if k.shape[0] == 1 else g_k
         g_s = g_s.sum(0, keepdim=True) if s.shape[0] == 1 else g_s
     return g_k, g_s
+
+
+_ray_setup_bwd_op = torch.library.custom_op("nanodrr_gb300::ray_setup_bwd", mutates_args=())(_ray_setup_bwd)
 
 
 @_ray_setup_bwd_op.register_fake
@@ -207,7 +214,8 @@ def _ray_setup_context(ctx, inputs, output):
 
 def _ray_setup_backward(ctx, gsrc, gtgt, gstep):
     k_inv, sdd = ctx.saved_tensors
-    g_k, g_s = _ray_setup_bwd_op(gsrc, gtgt, gstep, k_inv, sdd, *ctx.args)
+    bwd = _ray_setup_bwd if plain_eager(gsrc, gtgt, gstep, k_inv, sdd) else _ray_setup_bwd_op
+    g_k, g_s = bwd(gsrc, gtgt, gstep, k_inv, sdd, *ctx.args)
     return (g_k if ctx.needs_input_grad[0] else None, g_s if ctx.needs_input_grad[1] else None, *[None] * 5)
 
 
@@ -231,7 +239,7 @@ def _camera_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, low: bool) -> tuple[
     M_lo = torch.empty(B, 3, 4, device=rt.device) if low else M.new_empty(0)
     _ffi.check(_ffi.load().ndrr_camera_affine(w.data_ptr(), rt.data_ptr(), B, M.data_ptr(),
                                               M_lo.data_ptr() if low else None,
-                                              torch.cuda.current_stream(rt.device).cuda_stream), "ndrr_camera_affine")
+                                              _ffi.stream_handle(rt.device)), "ndrr_camera_affine")
     return M, M_lo
 
 
@@ -246,14 +254,17 @@ def _(w2v, rt_inv):
     return rt_inv.new_empty(rt_inv.shape[0], 3, 4), rt_inv.new_empty(rt_inv.shape[0], 3, 4)
 
 
-@torch.library.custom_op("nanodrr_gb300::camera_affine_bwd", mutates_args=())
-def _camera_affine_bwd_op(gM: torch.Tensor, w2v: torch.Tensor) -> torch.Tensor:
+def _camera_affine_bwd(gM: torch.Tensor, w2v: torch.Tensor) -> torch.Tensor:
     g, w = gM.contiguous(), w2v.contiguous()
     out = torch.empty(g.shape[0], 4, 4, device=g.device)
     _ffi.check(_ffi.load().ndrr_camera_affine_bwd(w.data_ptr(), g.data_ptr(), g.shape[0], out.data_ptr(),
-                                                  torch.cuda.current_stream(g.device).cuda_stream),
+                                                  _ffi.stream_handle(g.device)),
                "ndrr_camera_affine_bwd")
     return out
+
+
+_camera_affine_bwd_op = torch.library.custom_op("nanodrr_gb300::camera_affine_bwd",
+                                                mutates_args=())(_camera_affine_bwd)
 
 
 @_camera_affine_bwd_op.register_fake
@@ -270,7 +281,8 @@ def _camera_affine_backward(ctx, gM, _g_lo):
     # M_lo is a rounding correction of M, not differentiated
     if gM is None:
         return None, None
-    return None, _camera_affine_bwd_op(gM, ctx.saved_tensors[0])
+    w2v = ctx.saved_tensors[0]
+    return None, (_camera_affine_bwd if plain_eager(gM, w2v) else _camera_affine_bwd_op)(gM, w2v)
 
 
 torch.library.register_autograd("nanodrr_gb300::camera_affine", _camera_affine_backward,
@@ -295,14 +307,14 @@ def _call_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, grad: bool) -> torch.T
     if (grad or (hasattr(torch, "compiler") and torch.compiler.is_compiling())
             or rt_inv.device.type != "cuda" or torch.cuda.is_current_stream_capturing()):
         return product()
-    stream = torch.cuda.current_stream(rt_inv.device)
+    stream = _ffi.stream_handle(rt_inv.device)
     key = (id(w2v), id(rt_inv))
     hit = _M_CACHE.get(key)
     if hit is not None:
         wref, wver, rref, rver, M, made_on = hit
         if wref() is w2v and rref() is rt_inv and wver == w2v._version and rver == rt_inv._version:
             if stream != made_on:  # keep the allocator from reusing it under this stream's kernels
-                M.record_stream(stream)
+                M.record_stream(torch.cuda.current_stream(rt_inv.device))
             return M
     M = product()
     for k in [k for k, v in _M_CACHE.items() if v[0]() is None or v[2]() is None]:
@@ -330,6 +342,13 @@ def compact_label(subject: Subject) -> torch.Tensor:
     packed = torch.where((t >= 0) & (t < C), t, torch.full_like(t, 255.0)).to(torch.uint8).contiguous()
     object.__setattr__(subject, "_ndrr_label_cache", (key, packed))
     return packed
+
+
+def _batched(t: torch.Tensor, B: int) -> torch.Tensor:
+    """`t` expanded to B poses, float32 and contiguous (itself when it is)."""
+    if t.shape[0] == B and t.dtype == torch.float32 and t.is_contiguous():
+        return t
+    return t.expand(B, *[-1] * (t.dim() - 1)).float().contiguous()
 
 
 def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) -> torch.Tensor:
@@ -366,15 +385,15 @@ def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) 
         M = M.expand(B, -1, -1)
         if grad:
             M_lo = M_lo.expand(B, -1, -1)
-    if not fused_supported(subject, B, height * width):
+    if not _within_limits(img, C, B * height * width):
         raise ValueError("inputs exceed the CUDA kernel's limits (int32 indexing)")
     args = (
         vol,
         lab,
         M.contiguous(),
-        src.expand(B, -1, -1).float().contiguous(),
-        tgt.expand(B, -1, -1).float().contiguous(),
-        step_size.expand(B, -1).float().contiguous(),
+        _batched(src, B),
+        _batched(tgt, B),
+        _batched(step_size, B),
         n_samples,
         C,
         width,
@@ -395,8 +414,16 @@ def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) 
     # Without a recorded gradient the forward is called directly, skipping
     # the custom op's dispatch (tens of microseconds of host time per call).
     direct = not compiling and not grad
-    quad = cached_quad(subject, vol, lab, C) if layout == "quad" else vol.new_empty(0, dtype=torch.uint8)
+    quad = cached_quad(subject, vol, lab, C) if layout == "quad" else None
+    if direct:
+        sk = None
+        if skip is not None and int(skip.mode) != _ffi.NDRR_SKIP_NONE:
+            sk = _SkipArgs(skip.grid.grid, skip.grid.cell, skip.packed, int(skip.mode), float(skip.margin), vol.shape,
+                           getattr(skip, "fused", True))
+        return march_direct(vol, quad, *args[1:], skip=sk).reshape(B, C, height, width)
     empty = vol.new_empty(0, dtype=torch.uint8)
+    if quad is None:
+        quad = empty
     if skip is not None:
         # With a gradient recorded the skip always goes through sample windows
         # computed ahead of the march (not the in-kernel walk of a fused
@@ -408,8 +435,7 @@ def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) 
     else:
         sk = (empty, 0, empty, 0, 0.0, False)
     slab_mib = int(getattr(subject, "slab_mib", 0))
-    op = fused_raymarch_ex_forward if direct else fused_raymarch_ex
-    out = op(args[0], quad, args[1], args[2], M_lo.contiguous(), *args[3:], *sk, slab_mib)[0]
+    out = fused_raymarch_ex(args[0], quad, args[1], args[2], M_lo.contiguous(), *args[3:], *sk, slab_mib)[0]
     return out.reshape(B, C, height, width)
 
 
@@ -505,7 +531,7 @@ def _cached_rays(k_inv, sdd, height, width, n_samples, orthographic, rt_inv):
     device, dtype = rt_inv.device, rt_inv.dtype
     if device.type != "cuda" or torch.cuda.is_current_stream_capturing():
         return None
-    stream = torch.cuda.current_stream(device)
+    stream = _ffi.stream_handle(device)
     B = max(rt_inv.shape[0], k_inv.shape[0], sdd.shape[0])
     key = (id(k_inv), id(sdd), height, width, n_samples, bool(orthographic), B, dtype, device)
     hit = _RAY_CACHE.get(key)
@@ -514,7 +540,7 @@ def _cached_rays(k_inv, sdd, height, width, n_samples, orthographic, rt_inv):
         if kref() is k_inv and sref() is sdd and kver == k_inv._version and sver == sdd._version:
             if stream != made_on:  # keep the allocator from reusing them under this stream's kernels
                 for t in rays:
-                    t.record_stream(stream)
+                    t.record_stream(torch.cuda.current_stream(device))
             return rays
     if _ray_setup_takes(k_inv, sdd, height, width, rt_inv):
         rays = _ray_setup(k_inv, sdd, B, height, width, n_samples, bool(orthographic))

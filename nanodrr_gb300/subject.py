@@ -74,7 +74,7 @@ def hu_to_mu(data: torch.Tensor, mu_water=MU_WATER, mu_bone=MU_BONE, hu_bone=HU_
     out = torch.empty_like(src)
     if src.numel():
         lib = _ffi.load()
-        stream = torch.cuda.current_stream(src.device).cuda_stream
+        stream = _ffi.stream_handle(src.device)
         _ffi.check(
             lib.ndrr_hu_to_mu(ctypes.c_void_p(src.data_ptr()), ndrr_dtype(src), ctypes.c_int64(src.numel()),
                               ctypes.c_float(mu_water), ctypes.c_float(mu_bone), ctypes.c_float(hu_bone),
