@@ -271,10 +271,28 @@ enum ndrr_gvol_mode {
                                 slab order from sample positions alone (no
                                 gathers). Quad layout, one channel, no camera
                                 gradients (else NDRR_GVOL_SLAB); the workspace
-                                is NDRR_GVOL_SLAB's. Measured slower than
-                                NDRR_GVOL_SLAB (8.65 against 6.79 ms at 512^3,
-                                32 x 256^2): the scatter is the bound      */
+                                is NDRR_GVOL_SLAB's. 2.7 + 4.3 against 6.4 ms of
+                                NDRR_GVOL_SLAB at 512^3, 32 x 256^2: the two
+                                passes pay where the first is the forward
+                                (ndrr_raymarch_fwd_sums + _gvol)             */
 };
+
+/* A one-channel forward over the quad layout (vol_quad; out in the volume's
+ * dtype; sample_window allowed, no skip_mode) that also leaves, per ray, the
+ * sums the pose adjoint needs from the samples: sums [6, B, N] f32, sum dv
+ * and sum t dv over the samples' voxel-space position gradients.
+ * ndrr_pose_from_sums forms gM from them and go (args: go, src, tgt, step, gM
+ * and a workspace of ndrr_pose_from_sums_workspace_bytes) without marching
+ * the volume; deterministic. */
+NDRR_API int32_t ndrr_raymarch_fwd_sums(const ndrr_raymarch_args* a, float* sums, void* stream);
+NDRR_API int32_t ndrr_pose_from_sums_workspace_bytes(int32_t B, int32_t N, uint64_t* bytes);
+NDRR_API int32_t ndrr_pose_from_sums(const ndrr_raymarch_args* a, const float* sums, void* stream);
+
+/* The volume gradient alone (quad layout, one channel, need_gvol = 1, no camera
+ * gradients, gvol_mode NDRR_GVOL_AUTO or NDRR_GVOL_SLAB): a positions-only scatter
+ * in slab order; gM is not computed. The workspace is
+ * ndrr_raymarch_bwd_workspace_bytes'. */
+NDRR_API int32_t ndrr_raymarch_gvol(const ndrr_raymarch_args* a, void* stream);
 
 /* Library identity. */
 NDRR_API int32_t ndrr_abi_version(void);

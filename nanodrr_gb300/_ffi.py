@@ -174,6 +174,11 @@ SIGNATURES: dict[str, tuple] = {
     "ndrr_reduce_probe": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int32, _i32p, ctypes.c_void_p]),
     "ndrr_occupancy_dims": (ctypes.c_int32, [ctypes.c_int32] * 4 + [_i32p] * 3),
     "ndrr_occupancy_build": (ctypes.c_int32, [ctypes.POINTER(OccupancyArgs), ctypes.c_void_p]),
+    "ndrr_raymarch_fwd_sums": (ctypes.c_int32, [ctypes.POINTER(RaymarchArgs), ctypes.c_void_p, ctypes.c_void_p]),
+    "ndrr_pose_from_sums_workspace_bytes": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_int32,
+                                                             ctypes.POINTER(ctypes.c_uint64)]),
+    "ndrr_pose_from_sums": (ctypes.c_int32, [ctypes.POINTER(RaymarchArgs), ctypes.c_void_p, ctypes.c_void_p]),
+    "ndrr_raymarch_gvol": (ctypes.c_int32, [ctypes.POINTER(RaymarchArgs), ctypes.c_void_p]),
     "ndrr_skip_windows": (ctypes.c_int32, [ctypes.POINTER(RaymarchArgs), ctypes.c_void_p, ctypes.c_void_p]),
     "ndrr_texture_create": (ctypes.c_int32, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                              ctypes.POINTER(ctypes.c_uint64), ctypes.c_void_p]),

@@ -29,8 +29,8 @@ __global__ void __launch_bounds__(256) pose_partials_reduce_kernel(const float* 
     }
 }
 
-static cudaError_t launch_pose_reduce(const float* partials, int B, int tiles, float* gM, float* gsrc_shared,
-                                      cudaStream_t st) {
+cudaError_t launch_pose_reduce(const float* partials, int B, int tiles, float* gM, float* gsrc_shared,
+                               cudaStream_t st) {
     pose_partials_reduce_kernel<<<dim3((unsigned)B, gsrc_shared ? 15 : 12), 256, 0, st>>>(partials, tiles, gM,
                                                                                          gsrc_shared);
     return cudaGetLastError();
@@ -59,6 +59,15 @@ static cudaError_t bwd_dispatch(const MarchParams& p, bool multi, bool gvol, boo
                                 unsigned block, size_t smem, cudaStream_t st) {
     if (multi) return bwd_dispatch_flags<VT, true>(p, gvol, gcam, skip, grid, block, smem, st);
     return bwd_dispatch_flags<VT, false>(p, gvol, gcam, skip, grid, block, smem, st);
+}
+
+// The volume gradient alone (quad layout, one channel): positions-only scatter
+// in slab order and the fold.
+cudaError_t launch_gvol(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(a.gvol_quad, 0, (size_t)(a.D + 4) * (a.H + 3) * (a.W + 3) * 16, st);
+    if (e == cudaSuccess) e = launch_scatter_slab(a, ls, make_params(a, ls), st);
+    if (e == cudaSuccess) e = launch_quad_fold(a.gvol_quad, a.D, a.H, a.W, a.gvol, a.gvol_overwrite != 0, st);
+    return e;
 }
 
 cudaError_t launch_bwd(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaStream_t st) {

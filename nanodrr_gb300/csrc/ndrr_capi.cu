@@ -316,6 +316,74 @@ int32_t ndrr_raymarch_bwd(const ndrr_raymarch_args* a, void* stream) {
     return ok();
 }
 
+int32_t ndrr_raymarch_fwd_sums(const ndrr_raymarch_args* a, float* sums, void* stream) {
+    int32_t rc = validate_common(a);
+    if (rc != NDRR_OK) return rc;
+    if (a->B == 0 || a->N == 0) return ok();
+    if (a->out == nullptr || sums == nullptr || misaligned(sums, 4))
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "out and sums must be non-NULL and 4-byte aligned");
+    if (a->vol_quad == nullptr || a->n_classes != 1 || a->skip_mode != NDRR_SKIP_NONE || a->out_dtype != a->vol_dtype ||
+        a->fwd_mode != NDRR_FWD_DEFAULT || a->vol_texture != 0 || a->out_total != nullptr || a->out_extent != nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT,
+                    "the forward with pose sums takes one channel of the quad layout, output in the volume's dtype, no "
+                    "skip_mode, variant, total or extent output");
+    if (ndrr::wide_volume(a->D, a->H, a->W))
+        return fail(NDRR_ERR_LIMIT, "the forward with pose sums takes axes below 2^22 voxels");
+    ndrr::LaunchShape ls = ndrr::choose_shape(*a, sm_count_current());
+    ls.K = 1;
+    rc = validate_shape(ls, 0);
+    if (rc != NDRR_OK) return rc;
+    const cudaError_t e = ndrr::launch_fwd_sums(*a, ls, sums, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_pose_from_sums_workspace_bytes(int32_t B, int32_t N, uint64_t* bytes) {
+    if (bytes == nullptr || B < 0 || N < 0) return fail(NDRR_ERR_INVALID_ARGUMENT, "bad pose-sum shape");
+    *bytes = ndrr::pose_sums_workspace_bytes(B, N);
+    return ok();
+}
+
+int32_t ndrr_pose_from_sums(const ndrr_raymarch_args* a, const float* sums, void* stream) {
+    int32_t rc = validate_common(a);
+    if (rc != NDRR_OK) return rc;
+    if (a->B == 0 || a->N == 0) return ok();
+    if (a->go == nullptr || a->gM == nullptr || sums == nullptr)
+        return fail(NDRR_ERR_INVALID_ARGUMENT, "go, gM and sums must be non-NULL");
+    if (!is_float_dtype(a->go_dtype)) return fail(NDRR_ERR_DTYPE, "go dtype %d unsupported", a->go_dtype);
+    if (a->n_classes != 1) return fail(NDRR_ERR_INVALID_ARGUMENT, "pose sums are of one channel");
+    const uint64_t need = ndrr::pose_sums_workspace_bytes(a->B, a->N);
+    if (a->workspace == nullptr || a->workspace_bytes < need)
+        return fail(NDRR_ERR_WORKSPACE, "pose sums need %llu workspace bytes, got %llu", (unsigned long long)need,
+                    (unsigned long long)(a->workspace ? a->workspace_bytes : 0));
+    const cudaError_t e = ndrr::launch_pose_sums(*a, sums, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "pose sum launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
+int32_t ndrr_raymarch_gvol(const ndrr_raymarch_args* a, void* stream) {
+    int32_t rc = validate_common(a);
+    if (rc != NDRR_OK) return rc;
+    if (a->B == 0 || a->N == 0) return ok();
+    if (a->go == nullptr) return fail(NDRR_ERR_INVALID_ARGUMENT, "go is NULL");
+    if (!is_float_dtype(a->go_dtype)) return fail(NDRR_ERR_DTYPE, "go dtype %d unsupported", a->go_dtype);
+    if (a->vol_quad == nullptr || a->gvol_quad == nullptr || a->gvol == nullptr || a->need_gvol == 0 ||
+        a->need_gcam != 0 || a->n_classes != 1 || (a->gvol_mode != NDRR_GVOL_AUTO && a->gvol_mode != NDRR_GVOL_SLAB))
+        return fail(NDRR_ERR_INVALID_ARGUMENT,
+                    "the volume-gradient pass takes one channel of the quad layout with need_gvol, gvol and gvol_quad, "
+                    "gvol_mode 0 or 3 and no camera gradients");
+    const ndrr::LaunchShape ls = ndrr::choose_shape(*a, 0);
+    const uint64_t need = ndrr::bwd_workspace_bytes(*a, ls);
+    if (a->workspace == nullptr || a->workspace_bytes < need)
+        return fail(NDRR_ERR_WORKSPACE, "adjoint needs %llu workspace bytes, got %llu", (unsigned long long)need,
+                    (unsigned long long)(a->workspace ? a->workspace_bytes : 0));
+    rc = validate_shape(ls, 0);
+    if (rc != NDRR_OK) return rc;
+    const cudaError_t e = ndrr::launch_gvol(*a, ls, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail(NDRR_ERR_CUDA, "volume-gradient launch failed: %s", cudaGetErrorString(e));
+    return ok();
+}
+
 int32_t ndrr_skip_windows(const ndrr_raymarch_args* a, int32_t* windows, void* stream) {
     int32_t rc = validate_common(a);
     if (rc != NDRR_OK) return rc;

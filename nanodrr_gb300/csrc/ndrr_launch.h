@@ -8,6 +8,13 @@
 
 namespace ndrr {
 
+// A volume whose float voxel positions the forward's fast floor does not cover
+// (floor_frac): its forward takes the volume layout's converting loop.
+__host__ __device__ inline bool wide_volume(int D, int H, int W) {
+    constexpr int kWide = 1 << 22;
+    return D >= kWide || H >= kWide || W >= kWide;
+}
+
 struct LaunchShape {
     int tw = 16;  // tile width in rays (multiple of 8)
     int th = 8;   // tile height in rays (multiple of 4)
@@ -46,6 +53,10 @@ cudaError_t launch_fwd_tma(const ndrr_raymarch_args& a, const LaunchShape& ls, c
 cudaError_t texture_create(const float* vol, int D, int H, int W, unsigned long long* handle, cudaStream_t st);
 cudaError_t texture_destroy(unsigned long long handle, bool* known);
 cudaError_t launch_bwd(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaStream_t st);
+cudaError_t launch_gvol(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaStream_t st);
+cudaError_t launch_fwd_sums(const ndrr_raymarch_args& a, LaunchShape ls, float* sums, cudaStream_t st);
+uint64_t pose_sums_workspace_bytes(int B, int N);
+cudaError_t launch_pose_sums(const ndrr_raymarch_args& a, const float* sums, cudaStream_t st);
 uint64_t slab_workspace_bytes(const ndrr_raymarch_args& a, const LaunchShape& ls);
 float* slab_partials(const ndrr_raymarch_args& a, const LaunchShape& ls);
 int homography_blocks(int H, int W);

@@ -81,13 +81,6 @@ struct MarchParams {
     int tw, th, K;
 };
 
-// A volume whose float voxel positions the forward's fast floor does not cover
-// (floor_frac): its forward takes the volume layout's converting loop.
-__host__ __device__ __forceinline__ bool wide_volume(int D, int H, int W) {
-    constexpr int kWide = 1 << 22;
-    return D >= kWide || H >= kWide || W >= kWide;
-}
-
 constexpr int kSkipSteps = 256;  // distance-field steps per query before giving up
 
 constexpr int kPartialStride = 16;  // 12 pose terms + 3 shared-source terms + pad
@@ -1119,6 +1112,8 @@ cudaError_t launch_bwd_slab(const ndrr_raymarch_args& a, const LaunchShape& ls, 
 cudaError_t launch_scatter_slab(const ndrr_raymarch_args& a, const LaunchShape& ls, const MarchParams& p0,
                                 cudaStream_t st);
 size_t fwd_base_bytes(const ndrr_raymarch_args& a, const LaunchShape& ls);
+cudaError_t launch_pose_reduce(const float* partials, int B, int tiles, float* gM, float* gsrc_shared,
+                               cudaStream_t st);
 
 template <typename Kern>
 static cudaError_t launch_kernel(Kern kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st,

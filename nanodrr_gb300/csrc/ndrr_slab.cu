@@ -267,35 +267,130 @@ __global__ void __maxnreg__(96) raymarch_bwd_slab_kernel(const MarchParams p, co
 }
 
 // Volume-gradient scatter of one (slab, pose, tile) item from sample
-// positions alone: the split adjoint's second pass. The terms are those of
-// adjoint_accumulate's scatter (go * step * trilinear weight per corner, two
-// 16-byte reductions into the quad gradient per sample); the volume values
-// and the pose terms, which need the gathers, come from the first pass.
-__device__ __forceinline__ void scatter_body(const MarchParams& p, const int tile, const int b,
-                                             const SlabCut cut) {
-    const int n = tile_ray(p.tm, p.N, p.tw, p.th, tile, (int)threadIdx.x);
-    if (n < 0) return;
-    float m[12];
+// positions alone: the terms of adjoint_accumulate's scatter (go * step *
+// trilinear weight per corner) into the quad gradient, without volume values
+// or pose terms.
+//
+// A thread takes a column of NC rays (neighbours down the detector) at the same
+// sample index. Their cells are often the same or one above the other (the
+// spacing of the rays is about a voxel) and then share quad elements: the
+// shared terms are added in registers and reduced once. The kernel is bound by
+// L1's request path to the crossbar, which every reduction takes.
+struct ScatterRay {
+    FixPos f0, fd;
+    float g;  // go * step
+    int s0, s1;
+};
+
+__device__ __forceinline__ void red4(float* a, const float (&v)[4]) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]));
+}
+
+template <int NC>
+__device__ __forceinline__ void scatter_body(const MarchParams& p, const int tile, const int b, const SlabCut cut) {
+    const int cols = p.th / NC, q = (int)(threadIdx.x >> 3);
+    const int px = (tile % p.tm.tiles_x) * p.tw + (q / cols) * 8 + (int)(threadIdx.x & 7);
+    const int py = (tile / p.tm.tiles_x) * p.th + (q % cols) * NC;
+    ScatterRay ray[NC];
+    int s0 = INT_MAX, s1 = 0;
+    {
+        float m[12];
 #pragma unroll
-    for (int j = 0; j < 12; ++j) m[j] = __ldg(p.M + (size_t)b * 12 + j);
-    ThreadRay tr;
-    init_thread_ray(p, m, b, n, tr);
-    restrict_to_slab(p, tr, cut);
-    const float go = ld_any_f(p.go, p.go_dtype, tr.bn);
-    if (go == 0.f) return;  // every term is proportional to go
-    const float g = go * tr.stepv;
-    const QuadScatter sc{p.gquad, p.qg};
-    int s0 = tr.ray.lo, s1 = tr.ray.hi;
-    trim_inside(p, tr, s0, s1);
+        for (int j = 0; j < 12; ++j) m[j] = __ldg(p.M + (size_t)b * 12 + j);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const int n0 = (py + j) * p.tm.IW + px;
+            const int n = px < p.tm.IW && py + j < p.tm.IH && n0 < p.N ? n0 : -1;
+            ThreadRay tr;
+            init_thread_ray(p, m, b, n, tr);
+            restrict_to_slab(p, tr, cut);
+            int a = tr.ray.lo, e = tr.ray.hi;
+            const float go = n >= 0 ? ld_any_f(p.go, p.go_dtype, tr.bn) : 0.f;
+            if (go == 0.f) e = a;  // every term is proportional to go
+            trim_inside(p, tr, a, e);
+            if (a >= e) {
+                a = INT_MAX;
+                e = 0;
+            }
+            ray[j] = ScatterRay{tr.f0, tr.fd, go * tr.stepv, a, e};
+            s0 = min(s0, a);
+            s1 = max(s1, e);
+        }
+    }
+    if (s0 >= s1) return;
+    // in order of rising z, so that an element shared by neighbours is the
+    // lower one's upper plane
+    auto at = [](const ScatterRay& r, int s) {
+        const unsigned long long u = (unsigned)s;
+        return FixPos{(long long)((unsigned long long)r.f0.x + u * (unsigned long long)r.fd.x),
+                      (long long)((unsigned long long)r.f0.y + u * (unsigned long long)r.fd.y),
+                      (long long)((unsigned long long)r.f0.z + u * (unsigned long long)r.fd.z)};
+    };
+    if (NC > 1 && at(ray[NC - 1], (s0 + s1) >> 1).z < at(ray[0], (s0 + s1) >> 1).z) {
+#pragma unroll
+        for (int j = 0; j < NC / 2; ++j) {
+            const ScatterRay t = ray[j];
+            ray[j] = ray[NC - 1 - j];
+            ray[NC - 1 - j] = t;
+        }
+    }
+    float* r0p = p.gquad;
+    float* r1p = p.gquad + (size_t)p.qg.plane * 4;
     for (int s = s0; s < s1; ++s) {
-        Cell c;
-        fix_cell(fix_at(tr, s), p.qg, c);
-        const float wy0 = 1.f - c.fy, wz0 = 1.f - c.fz;
-        sc(c, g * wz0 * wy0, g * wz0 * c.fy, g * c.fz * wy0, g * c.fz * c.fy, 1.f - c.fx, c.fx);
+        int qi = -1;  // element of the terms held back: lower plane, upper plane
+        float lo[4], hi[4];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const ScatterRay& r = ray[j];
+            if (s < r.s0 || s >= r.s1) continue;
+            Cell c;
+            fix_cell(at(r, s), p.qg, c);
+            const float wx0 = 1.f - c.fx, wy0 = 1.f - c.fy, wz0 = 1.f - c.fz;
+            const float g00 = r.g * wz0 * wy0, g01 = r.g * wz0 * c.fy, g10 = r.g * c.fz * wy0, g11 = r.g * c.fz * c.fy;
+            float l[4] = {g00 * wx0, g00 * c.fx, g01 * wx0, g01 * c.fx};
+            float h[4] = {g10 * wx0, g10 * c.fx, g11 * wx0, g11 * c.fx};
+            if (NC > 1 && qi >= 0) {
+                if (c.qi == qi) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        l[k] += lo[k];
+                        h[k] += hi[k];
+                    }
+                } else {
+                    red4(r0p + (size_t)(unsigned)qi * 4, lo);
+                    if (c.qi == qi + p.qg.plane) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) l[k] += hi[k];
+                    } else {
+                        red4(r1p + (size_t)(unsigned)qi * 4, hi);
+                    }
+                }
+            }
+            qi = c.qi;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                lo[k] = l[k];
+                hi[k] = h[k];
+            }
+        }
+        if (qi >= 0) {
+            red4(r0p + (size_t)(unsigned)qi * 4, lo);
+            red4(r1p + (size_t)(unsigned)qi * 4, hi);
+        }
     }
 }
 
-__global__ void __launch_bounds__(512) raymarch_scatter_slab_kernel(const MarchParams p, const SlabParams s) {
+// Registers by rays per thread (512^3, 32 poses x 256^2 x 800; 277 x 250 x 301, 9
+// poses x 211 x 187 x 383, kernel alone, ms): one ray at 80 registers 5.64 and
+// 0.409; two at 96 4.67 and 0.395 (0.450 at 72); four at 168 4.34 and 0.471.
+template <int NC>
+struct ScatterRegs {
+    static constexpr int value = NC == 1 ? 80 : NC == 2 ? 96 : 168;
+};
+
+template <int NC>
+__global__ void __maxnreg__(ScatterRegs<NC>::value) raymarch_scatter_slab_kernel(const MarchParams p, const SlabParams s) {
     __shared__ int item_sh;
     const int total = s.counters[0];
     while (true) {
@@ -309,7 +404,7 @@ __global__ void __launch_bounds__(512) raymarch_scatter_slab_kernel(const MarchP
         const int b = bt / p.tm.tiles, tile = bt % p.tm.tiles;
         const int axis = s.axis[b];
         const int thick = axis == 0 ? s.Z[0] : (axis == 1 ? s.Z[1] : s.Z[2]);
-        scatter_body(p, tile, b, SlabCut{axis, k * thick, (k + 1) * thick});
+        scatter_body<NC>(p, tile, b, SlabCut{axis, k * thick, (k + 1) * thick});
     }
 }
 
@@ -417,14 +512,22 @@ cudaError_t launch_scatter_slab(const ndrr_raymarch_args& a, const LaunchShape& 
     SlabParams s;
     cudaError_t e = slab_setup(a, ls, p, s, st);
     if (e != cudaSuccess) return e;
-    const int block = p.tw * p.th;
+    const int R = p.tw * p.th;
+    // Rays per thread: columns of four where the launch has rays enough to fill
+    // the GPU four times over with them (about 2^18 resident rays at 12 warps per
+    // SM), else of two, where the tile splits into whole warps of them.
+    const long long rays = (long long)a.B * a.N;
+    const int nc = rays >= (1 << 20) && R % 128 == 0 ? 4 : R % 64 == 0 ? 2 : 1;
+    auto kern = nc == 4 ? raymarch_scatter_slab_kernel<4>
+                        : nc == 2 ? raymarch_scatter_slab_kernel<2> : raymarch_scatter_slab_kernel<1>;
+    const int block = R / nc;
     int dev = 0, sms = 0, per_sm = 0;
     e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raymarch_scatter_slab_kernel, block, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)std::max(1, sms * std::max(per_sm, 1));
-    raymarch_scatter_slab_kernel<<<grid, block, 0, st>>>(p, s);
+    kern<<<grid, block, 0, st>>>(p, s);
     return cudaGetLastError();
 }
 

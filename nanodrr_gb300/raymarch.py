@@ -521,6 +521,37 @@ def raymarch_backward(
     return gvol, gM, gsrc, gtgt, gstep
 
 
+def volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo=None, slab_mib=0) -> torch.Tensor:
+    """The volume gradient alone of a one-channel render (float32 [D, H, W]):
+    a scatter from sample positions, without the volume's values and the pose
+    terms `raymarch_backward` computes with it."""
+    _check_inputs(vol, vol, M, src, tgt, step, n_samples, 1)
+    vol, _, M, src, tgt, step = _prep(vol, vol, M, src, tgt, step)
+    go = go.contiguous() if go.dtype in _FLOAT_DTYPES else go.float().contiguous()
+    if go.shape != (tgt.shape[0], 1, tgt.shape[1]):
+        raise ValueError(f"go must be [B, 1, N] = [{tgt.shape[0]}, 1, {tgt.shape[1]}], got {tuple(go.shape)}")
+    D, H, W = vol.shape
+    dev = vol.device
+    if tgt.shape[0] == 0 or tgt.shape[1] == 0:
+        return torch.zeros(vol.shape, device=dev, dtype=torch.float32)
+    a = _base_args(vol, vol, M, src, tgt, step, n_samples, 1, width)
+    _set_M_lo(a, M_lo, M)
+    gvol = torch.empty(vol.shape, device=dev, dtype=torch.float32)
+    gq = torch.empty((D + 4) * (H + 3) * (W + 3) * 4, device=dev, dtype=torch.float32)
+    a.go, a.go_dtype = _ptr(go), ndrr_dtype(go)
+    a.need_gvol, a.gvol_overwrite = 1, 1
+    a.gvol, a.gvol_quad, a.vol_quad = _ptr(gvol), gq.data_ptr(), quad.data_ptr()
+    quad_is_labeled(vol, quad)  # raises unless it is a quad copy of this volume
+    a.slab_mib = int(slab_mib)
+    lib = _ffi.load()
+    nbytes = ctypes.c_uint64(0)
+    _ffi.check(lib.ndrr_raymarch_bwd_workspace_bytes(ctypes.byref(a), ctypes.byref(nbytes)), "workspace query")
+    ws = torch.empty(max(int(nbytes.value), 16), device=dev, dtype=torch.uint8)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    _ffi.check(lib.ndrr_raymarch_gvol(ctypes.byref(a), _stream_handle(dev)), "ndrr_raymarch_gvol")
+    return gvol
+
+
 # --------------------------------------------------------------- custom ops
 @torch.library.custom_op("nanodrr_gb300::fused_raymarch", mutates_args=())
 def fused_raymarch(
@@ -722,12 +753,16 @@ def _ex_bwd(
     margin: float,
     windows: torch.Tensor,
     slab_mib: int,
+    need_gM: bool = True,
 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     if need_gvol and torch.are_deterministic_algorithms_enabled():
         raise RuntimeError(
             "Volume gradients on the cuda backend use nondeterministic atomics; "
             "disable deterministic algorithms or detach the volume"
         )
+    if need_gvol and not (need_gM or need_gcam) and n_classes == 1 and quad.numel():
+        none = [torch.empty(0, device=vol.device) for _ in range(4)]
+        return volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo, slab_mib), *none
     if windows.numel():
         skip, win = None, windows
     else:
@@ -742,9 +777,11 @@ fused_raymarch_ex_bwd = torch.library.custom_op("nanodrr_gb300::fused_raymarch_e
 
 
 @fused_raymarch_ex_bwd.register_fake
-def _(go, vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam, *rest):
+def _(go, vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam, occ_grid,
+      occ_cell, proposal, skip_mode, margin, windows, slab_mib, need_gM=True):
     B, N, _ = tgt.shape
-    gM = torch.empty(B, 3, 4, device=M.device, dtype=torch.float32)
+    alone = need_gvol and not (need_gM or need_gcam) and n_classes == 1 and quad.numel() > 0
+    gM = torch.empty((0,) if alone else (B, 3, 4), device=M.device, dtype=torch.float32)
     empty = gM.new_empty(0)
     gvol = torch.empty(vol.shape, device=M.device, dtype=torch.float32) if need_gvol else empty
     gsrc = torch.empty(src.shape, device=M.device, dtype=torch.float32) if need_gcam else empty
@@ -766,18 +803,18 @@ def _ex_backward(ctx, go, _gwin):
         return (None,) * 18
     vol, quad, lab, M, M_lo, src, tgt, step, occ_grid, proposal, windows = ctx.saved_tensors
     n_samples, n_classes, width, occ_cell, mode, margin, slab_mib = ctx.args
-    need_gvol = ctx.needs_input_grad[0]
+    need_gvol, need_gM = ctx.needs_input_grad[0], ctx.needs_input_grad[3]
     need_gcam = any(ctx.needs_input_grad[i] for i in (5, 6, 7))
     bwd = _ex_bwd if plain_eager(go, vol, M, src, tgt, step) else fused_raymarch_ex_bwd
     gvol, gM, gsrc, gtgt, gstep = bwd(
         go, vol, quad, lab, M, M_lo, src, tgt, step, n_samples, n_classes, width, need_gvol, need_gcam,
-        occ_grid, occ_cell, proposal, mode, margin, windows, slab_mib,
+        occ_grid, occ_cell, proposal, mode, margin, windows, slab_mib, need_gM,
     )
     return (
         gvol.to(vol.dtype) if need_gvol else None,
         None,  # quad: a derived copy of vol
         None,  # lab
-        gM.to(M.dtype),
+        gM.to(M.dtype) if need_gM else None,
         None,  # M_lo: a rounding correction of M, not differentiated
         gsrc.to(src.dtype) if need_gcam else None,
         gtgt.to(tgt.dtype) if need_gcam else None,
@@ -787,3 +824,110 @@ def _ex_backward(ctx, go, _gwin):
 
 
 torch.library.register_autograd("nanodrr_gb300::fused_raymarch_ex", _ex_backward, setup_context=_ex_setup_context)
+
+
+# ------------------------------------------------- large pose renders
+# The forward leaves the per-ray sums that the pose adjoint needs
+# (ndrr_raymarch_fwd_sums), so a backward to the pose reads 24 bytes per ray
+# instead of marching the volume again, and one to the volume too only
+# scatters. One channel, quad layout, no camera gradients.
+@torch.library.custom_op("nanodrr_gb300::fused_raymarch_sums", mutates_args=())
+def fused_raymarch_sums(
+    vol: torch.Tensor,
+    quad: torch.Tensor,
+    M: torch.Tensor,
+    M_lo: torch.Tensor,
+    src: torch.Tensor,
+    tgt: torch.Tensor,
+    step: torch.Tensor,
+    n_samples: int,
+    width: int,
+    occ_grid: torch.Tensor,
+    occ_cell: int,
+    proposal: torch.Tensor,
+    skip_mode: int,
+    margin: float,
+    slab_mib: int,
+) -> tuple[torch.Tensor, torch.Tensor]:
+    """(out [B, 1, N], sums [6, B, N]); the skip arguments as in
+    `fused_raymarch_ex`, always applied through sample windows."""
+    _check_inputs(vol, vol, M, src, tgt, step, n_samples, 1)
+    vol, _, M, src, tgt, step = _prep(vol, vol, M, src, tgt, step)
+    B, N, _ = tgt.shape
+    out = torch.empty(B, 1, N, device=vol.device, dtype=vol.dtype)
+    sums = torch.empty(6, B, N, device=vol.device, dtype=torch.float32)
+    a = _base_args(vol, vol, M, src, tgt, step, n_samples, 1, width)
+    _set_M_lo(a, M_lo, M)
+    a.out, a.out_dtype = _ptr(out), a.vol_dtype
+    a.vol_quad = quad.data_ptr()
+    quad_is_labeled(vol, quad)
+    skip = _skip_of(vol, occ_grid, occ_cell, proposal, skip_mode, margin)
+    windows = skip_windows(vol, M, src, tgt, step, n_samples, width, skip) if skip is not None else None
+    a.sample_window = _ptr(windows)
+    _ffi.check(_ffi.load().ndrr_raymarch_fwd_sums(ctypes.byref(a), _ptr(sums), _stream_handle(vol.device)),
+               "ndrr_raymarch_fwd_sums")
+    return out, sums
+
+
+@fused_raymarch_sums.register_fake
+def _(vol, quad, M, M_lo, src, tgt, step, n_samples, width, occ_grid, occ_cell, proposal, skip_mode, margin, slab_mib):
+    B, N, _ = tgt.shape
+    return vol.new_empty(B, 1, N), vol.new_empty(6, B, N, dtype=torch.float32)
+
+
+def _sums_bwd(go: torch.Tensor, vol: torch.Tensor, quad: torch.Tensor, M: torch.Tensor, M_lo: torch.Tensor,
+              src: torch.Tensor, tgt: torch.Tensor, step: torch.Tensor, sums: torch.Tensor, n_samples: int,
+              width: int, need_gvol: bool, slab_mib: int) -> tuple[torch.Tensor, torch.Tensor]:
+    if need_gvol and torch.are_deterministic_algorithms_enabled():
+        raise RuntimeError(
+            "Volume gradients on the cuda backend use nondeterministic atomics; "
+            "disable deterministic algorithms or detach the volume"
+        )
+    go = go.contiguous() if go.dtype in _FLOAT_DTYPES else go.float().contiguous()
+    B, N, _ = tgt.shape
+    dev = vol.device
+    gM = torch.empty(B, 3, 4, device=dev, dtype=torch.float32)
+    a = _base_args(vol, vol, M, src, tgt, step, n_samples, 1, width)
+    a.go, a.go_dtype, a.gM = _ptr(go), ndrr_dtype(go), _ptr(gM)
+    lib = _ffi.load()
+    nbytes = ctypes.c_uint64(0)
+    _ffi.check(lib.ndrr_pose_from_sums_workspace_bytes(B, N, ctypes.byref(nbytes)), "workspace query")
+    ws = torch.empty(max(int(nbytes.value), 16), device=dev, dtype=torch.uint8)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    _ffi.check(lib.ndrr_pose_from_sums(ctypes.byref(a), _ptr(sums), _stream_handle(dev)), "ndrr_pose_from_sums")
+    if not need_gvol:
+        return torch.empty(0, device=dev), gM
+    return volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo, slab_mib), gM
+
+
+_sums_bwd_op = torch.library.custom_op("nanodrr_gb300::fused_raymarch_sums_bwd", mutates_args=())(_sums_bwd)
+
+
+@_sums_bwd_op.register_fake
+def _(go, vol, quad, M, M_lo, src, tgt, step, sums, n_samples, width, need_gvol, slab_mib):
+    gvol = torch.empty(vol.shape if need_gvol else (0,), device=M.device, dtype=torch.float32)
+    return gvol, torch.empty(M.shape[0], 3, 4, device=M.device, dtype=torch.float32)
+
+
+def _sums_setup_context(ctx, inputs, output):
+    vol, quad, M, M_lo, src, tgt, step, n_samples, width = inputs[:9]
+    ctx.save_for_backward(vol, quad, M.contiguous(), M_lo, src, tgt, step, output[1])
+    ctx.args = (n_samples, width)
+    ctx.slab_mib = inputs[14]
+    ctx.set_materialize_grads(False)
+
+
+def _sums_backward(ctx, go, _g_sums):
+    if go is None:
+        return (None,) * 15
+    vol, quad, M, M_lo, src, tgt, step, sums = ctx.saved_tensors
+    if any(ctx.needs_input_grad[i] for i in (4, 5, 6)):
+        raise RuntimeError("fused_raymarch_sums has no camera gradients; use fused_raymarch_ex")
+    need_gvol = ctx.needs_input_grad[0]
+    bwd = _sums_bwd if plain_eager(go, vol, M, src, tgt, step) else _sums_bwd_op
+    gvol, gM = bwd(go, vol, quad, M, M_lo, src, tgt, step, sums, *ctx.args, need_gvol, ctx.slab_mib)
+    return (gvol.to(vol.dtype) if need_gvol else None, None, gM.to(M.dtype), *[None] * 12)
+
+
+torch.library.register_autograd("nanodrr_gb300::fused_raymarch_sums", _sums_backward,
+                                setup_context=_sums_setup_context)
