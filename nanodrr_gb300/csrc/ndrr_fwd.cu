@@ -37,14 +37,22 @@ static cudaError_t fwd_dispatch_out(const MarchParams& p, int out_dtype, bool mu
     }
 }
 
-cudaError_t launch_fwd(const ndrr_raymarch_args& a, const LaunchShape& ls, cudaStream_t st) {
+cudaError_t launch_fwd(const ndrr_raymarch_args& a, const LaunchShape& shape, cudaStream_t st) {
+    LaunchShape ls = shape;
     MarchParams p = make_params(a, ls);
+    const bool quad = a.vol_quad != nullptr && !p.wide;
+    if (!quad && a.tile_w == 0 && a.tile_h == 0 && ls.tw == 8 && ls.th == 4) {
+        // a small launch's one-warp tiles take the wide patch's shape
+        ls.tw = 16;
+        ls.th = 2;
+        p = make_params(a, ls);
+    }
     unsigned grid = (unsigned)((size_t)a.B * p.tm.tiles);
     const unsigned block = (unsigned)(ls.tw * ls.th * ls.K);
     const size_t smem = fwd_smem_bytes(a, ls);
     const bool multi = a.n_classes > 1;
     const int skip = a.skip_mode;
-    if (a.vol_quad != nullptr && !p.wide) {
+    if (quad) {
         if (a.out_dtype != a.vol_dtype) return cudaErrorNotSupported;
         return launch_fwd_quad(p, a.vol_dtype, multi, skip, a.quad_labels != 0, grid, block, smem, st);
     }

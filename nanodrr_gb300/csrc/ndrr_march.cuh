@@ -314,7 +314,8 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
     const int NT = R * p.K;
     const int tid = threadIdx.x;
     const int r = tid % R, k = tid / R;
-    const int n = tile_ray(p.tm, p.N, p.tw, p.th, tile, r);
+    const int pw = QUAD == kLayoutVolume ? wide_patch(p.tw, p.th) : 8;
+    const int n = tile_ray(p.tm, p.N, p.tw, p.th, tile, r, pw);
 
     float m[12];
 #pragma unroll
@@ -469,7 +470,7 @@ __device__ __forceinline__ void fwd_body(const MarchParams& p, const int tile, c
         // channel, so stores coalesce along the detector rows.
         for (int idx = tid; idx < R * p.C; idx += NT) {
             const int rr = idx % R, c = idx / R;
-            const int nn = tile_ray(p.tm, p.N, p.tw, p.th, tile, rr);
+            const int nn = tile_ray(p.tm, p.N, p.tw, p.th, tile, rr, pw);
             if (nn < 0) continue;
             float sum = smem[(size_t)c * NT + rr];
             for (int j = 1; j < p.K; ++j) sum += smem[(size_t)c * NT + rr + j * R];

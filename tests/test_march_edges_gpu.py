@@ -95,3 +95,29 @@ def test_a_target_far_outside():
         gM = raymarch_backward(go, vol, vol, _identity(), src, tgt, step, 9, 1, 0, False, False, quad=quad)[1]
         want = march_numpy_adjoint(go.cpu(), vol.cpu(), None, _identity().cpu(), src.cpu(), tgt.cpu(), step.cpu(), 9)[1]
         assert np.abs(gM.double().cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("C", [1, 3])
+@pytest.mark.parametrize("hw", [(1, 1), (3, 5), (2, 16), (5, 17), (33, 31)])
+@pytest.mark.parametrize("tile", [(0, 0), (8, 4), (16, 8), (24, 4), (32, 8)])
+def test_warp_patches_cover_the_detector(tile, hw, C):
+    """Every ray of the volume layout's forward, for each patch width, tile
+    remainder and channel count, bitwise the image of one ray a call."""
+    H, W = hw
+    g = torch.Generator().manual_seed(5)
+    vol = (torch.rand(SHAPE, generator=g) + 0.5).cuda()
+    lab = torch.randint(0, C, SHAPE, generator=g).float().cuda() if C > 1 else vol
+    y, x = torch.meshgrid(torch.linspace(0.3, 8.4, H), torch.linspace(0.2, 10.6, W), indexing="ij")
+    tgt = torch.stack([x, y, torch.full_like(x, 8.2)], -1).reshape(1, -1, 3).cuda()
+    src = torch.tensor([5.1, 3.9, -6.0], device="cuda").expand_as(tgt).contiguous()
+    step = ((tgt - src).norm(dim=-1) / 39).contiguous()
+    args = (vol, lab, _identity())
+    out, _ = raymarch_forward(*args, src, tgt, step, 40, C, W, tile=(*tile, 2))
+    if C == 1:
+        ref = march_numpy(vol.cpu(), None, _identity().cpu(), src.cpu(), tgt.cpu(), step.cpu(), 40)
+        # float32 positions up to 13 voxels: 1e-6 voxel each, values up to 1.5
+        assert np.abs(out.double().cpu().numpy() - ref).max() <= 1e-5 * max(1.0, np.abs(ref).max())
+    for n in range(0, H * W, max(1, H * W // 16)):
+        one = [t[:, n : n + 1].contiguous() for t in (src, tgt, step)]
+        o, _ = raymarch_forward(*args, *one, 40, C, 1, tile=(0, 0, 2))
+        assert torch.equal(o[..., 0], out[..., n])
