@@ -13,7 +13,7 @@
 // Both marches wait for the same gathers, so the one that does both costs about
 // what the adjoint alone does (kernels alone): 16 poses x 200^2 x 500 samples of
 // 512 x 512 x 400 f32 0.74 ms for 0.69 + 0.73, 8 poses x 1024^2 x 1000 with
-// occupancy windows 6.8 for 3.4 + 6.1.
+// occupancy windows 6.5 for 3.4 + 6.1.
 #include "ndrr_march.cuh"
 
 namespace ndrr {
@@ -34,10 +34,11 @@ __device__ __forceinline__ void cell_grad_shared(const Cell& c, float& gx, float
     gz = fmaf(c.fx, xz, fmaf(c.fy, y1 - y0, c.v100 - c.v000));
 }
 
-// 80 registers: 0.74 and 6.79 ms at the sizes above, 2.70 for 32 poses x 256^2 x
-// 800 of 512^3; 64 spill (0.82, 6.98, 3.24).
+// 96 registers: 0.74 and 6.52 ms at the sizes above, 2.62 for 32 poses x 256^2 x
+// 800 of 512^3; 80: 0.75, 6.64, 2.68; 72: 0.75, 6.65, 2.70; 64 spill. Three
+// samples in flight at 112: 0.80, 6.76, 2.78.
 template <typename VT>
-__global__ void __maxnreg__(80) raymarch_fwd_sums_kernel(const MarchParams p, float* __restrict__ sums) {
+__global__ void __maxnreg__(96) raymarch_fwd_sums_kernel(const MarchParams p, float* __restrict__ sums) {
     const int tile = (int)(blockIdx.x % (unsigned)p.tm.tiles), b = (int)(blockIdx.x / (unsigned)p.tm.tiles);
     const int n = tile_ray(p.tm, p.N, p.tw, p.th, tile, threadIdx.x);
     if (n < 0) return;
@@ -48,10 +49,10 @@ __global__ void __maxnreg__(80) raymarch_fwd_sums_kernel(const MarchParams p, fl
         for (int j = 0; j < 12; ++j) m[j] = __ldg(p.M + (size_t)b * 12 + j);
         init_thread_ray(p, m, b, n, tr);
     }
-    // offset of float position p0 + t d from the cell corner i
-    auto offset = [](float t, float d, float p0, int i) {
-        return fmaf(t, d, p0) - (__uint_as_float(kFloorBits + (unsigned)i) - kFloorMagic);
-    };
+    // Offset of float position p0 + t d from the cell corner i. The march is
+    // bound by issue (73 % of slots) and the conversion pipe is idle, so i is
+    // converted: two instructions where forming it from bits took three.
+    auto offset = [](float t, float d, float p0, int i) { return fmaf(t, d, p0) - (float)i; };
     int s = tr.ray.lo, s1 = tr.ray.hi;
     trim_inside(p, tr, s, s1);
     float acc = 0.f, G[3] = {0.f, 0.f, 0.f}, Gt[3] = {0.f, 0.f, 0.f};
