@@ -546,7 +546,7 @@ __device__ __forceinline__ int tile_ray(const TileMap& m, int N, int tw, int th,
 
 // Patch width of the volume-layout forward's warps. It waits on L1 wavefronts
 // (92 % busy: eight scalar gathers a sample), and a wider row of neighbouring
-// rays shares more of each line: 200^2 x 500 frames of a 256^3 volume took
+// rays shares more of each line: 200^2 x 500 frames of 512 x 512 x 400 took
 // 86-100 us with 8 x 4 patches, 74-89 with 16 x 2 and 96-105 with 32 x 1
 // (float16 99-110, 84-98, 98-104; 128^2 42-47, 42-47, 42-49). The quad layout
 // reads 16 bytes a gather and keeps 8 x 4 (512^3 x 32 poses 1373 us, 1399 with
