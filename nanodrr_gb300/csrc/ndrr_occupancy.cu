@@ -28,11 +28,16 @@ namespace ndrr {
 // per cell plane in shared memory; a cell is occupied when any line of its y
 // range has a bit in its x range. Reading each cell's (cell + 4)^3 voxels per
 // thread took 325 us at 512 x 512 x 400 (cell 4, every voxel read eight times
-// through L1), this 196: every voxel is read 1.6 times, once from DRAM (62 us
-// at copy speed).
+// through L1), this 142: every voxel is read 1.9 times, once from DRAM (62 us
+// at copy speed). Tiles of 16 lines give CTAs enough for eight an SM in whole
+// waves; with 64 lines (1.6 reads) and four voxel planes in flight, not six, it
+// was 196. Six planes are half of a cell pair's twelve; 32 lines 144, 8 lines
+// 145, 3 planes 153, 12 planes 160, four cell planes a CTA 182-195.
 constexpr int kOccThreads = 256;
 constexpr int kOccPlanes = 2;   // cell planes per CTA
-constexpr int kOccLines = 64;   // volume lines of a tile's cells (without the two-voxel margins)
+constexpr int kOccLines = 16;   // volume lines of a tile's cells (without the two-voxel margins); one cell if larger
+constexpr int kOccMaxCell = 64;
+constexpr int kOccBatch = 6;    // voxel planes in flight
 constexpr int kOccSpan = 1024;  // voxels in x of a tile's cells (without the margins)
 constexpr int kOccWords = (kOccSpan / 128 + 2) * 4;
 
@@ -64,7 +69,7 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const VT* __rest
                                                                 int cell, int gx, int gy, int gz, int ty, int tx,
                                                                 int tiles_y, int tiles_x, uint8_t* __restrict__ dist,
                                                                 int max_dist) {
-    __shared__ unsigned bits[kOccPlanes][kOccLines + 4][kOccWords];
+    __shared__ unsigned bits[kOccPlanes][kOccMaxCell + 4][kOccWords];
     const int tile = (int)(blockIdx.x % (unsigned)(tiles_x * tiles_y));
     const int cz0 = (int)(blockIdx.x / (unsigned)(tiles_x * tiles_y)) * kOccPlanes;
     const int cy0 = (tile / tiles_x) * ty, cx0 = (tile % tiles_x) * tx;
@@ -89,12 +94,12 @@ __global__ void __launch_bounds__(kOccThreads) occupancy_kernel(const VT* __rest
 #pragma unroll
         for (int k = 0; k < kOccPlanes; ++k) m[k] = 0u;
         int z = zlo[0];
-        for (; z + 3 <= zhi[kOccPlanes - 1]; z += 4, p += 4 * plane) {
-            unsigned v[4];
+        for (; z + kOccBatch - 1 <= zhi[kOccPlanes - 1]; z += kOccBatch, p += kOccBatch * plane) {
+            unsigned v[kOccBatch];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = nonzero4<VT, VEC>(p + j * plane, x, W);
+            for (int j = 0; j < kOccBatch; ++j) v[j] = nonzero4<VT, VEC>(p + j * plane, x, W);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < kOccBatch; ++j)
 #pragma unroll
                 for (int k = 0; k < kOccPlanes; ++k)
                     if (z + j >= zlo[k] && z + j <= zhi[k]) m[k] |= v[j];
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(256) distance_axis_kernel(const uint8_t* __res
 template <typename VT>
 static cudaError_t occupancy(const void* vol, int D, int H, int W, int cell, int gx, int gy, int gz, int max_dist,
                              uint8_t* dist, cudaStream_t st) {
-    const int ty = kOccLines / cell, tx = kOccSpan / cell;  // cell <= 64
+    const int ty = std::max(1, kOccLines / cell), tx = kOccSpan / cell;  // cell <= kOccMaxCell
     const int tiles_y = (gy + ty - 1) / ty, tiles_x = (gx + tx - 1) / tx;
     const long long grid = (long long)tiles_y * tiles_x * ((gz + kOccPlanes - 1) / kOccPlanes);
     const bool vec = W % 4 == 0 && (uintptr_t)vol % (4 * sizeof(VT)) == 0;  // vector loads of four voxels

@@ -74,3 +74,14 @@ def _grid(v, cell, max_dist, shape):
         return eso.occupancy_grid(v, cell, max_dist)
     d = eso.occupancy_grid(v, cell, near).astype(np.int64)
     return np.where(d == near, max_dist, d).astype(np.uint8)
+
+
+@pytest.mark.parametrize("cell", [5, 8, 9, 16, 17, 33])
+@pytest.mark.parametrize("shape", [(13, 35, 40), (37, 18, 131)])
+def test_occupancy_around_the_tile_height(shape, cell):
+    """Cells that tile the CTA's lines with a remainder, fill them and exceed them."""
+    rng = np.random.default_rng(cell + 1)
+    for density in (1e-4, 1e-2):
+        v = np.where(rng.random(shape) < density, 1.0, 0.0).astype(np.float32)
+        got = OccupancyGrid.build(torch.from_numpy(v).cuda(), cell=cell, max_dist=4).grid.cpu().numpy()
+        assert np.array_equal(got, _grid(v, cell, 4, got.shape))
