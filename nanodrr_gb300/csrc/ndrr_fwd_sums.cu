@@ -34,9 +34,10 @@ __device__ __forceinline__ void cell_grad_shared(const Cell& c, float& gx, float
     gz = fmaf(c.fx, xz, fmaf(c.fy, y1 - y0, c.v100 - c.v000));
 }
 
-// 96 registers: 0.74 and 6.52 ms at the sizes above, 2.62 for 32 poses x 256^2 x
-// 800 of 512^3; 80: 0.75, 6.64, 2.68; 72: 0.75, 6.65, 2.70; 64 spill. Three
-// samples in flight at 112: 0.80, 6.76, 2.78.
+// Register cap 96 (71 used, seven CTAs an SM): 0.74 and 6.52 ms at the sizes above,
+// 2.62 for 32 poses x 256^2 x 800 of 512^3; scheduled under a cap of 80: 0.75, 6.64,
+// 2.68; of 72: 0.75, 6.65, 2.70; 64 spill. Three samples in flight at 112: 0.80,
+// 6.76, 2.78.
 template <typename VT>
 __global__ void __maxnreg__(96) raymarch_fwd_sums_kernel(const MarchParams p, float* __restrict__ sums) {
     const int tile = (int)(blockIdx.x % (unsigned)p.tm.tiles), b = (int)(blockIdx.x / (unsigned)p.tm.tiles);
