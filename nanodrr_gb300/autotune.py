@@ -88,8 +88,8 @@ class Autotuner:
         if k in self.cache:
             return int(self.cache[k][0])
         lab = vol if lab is None else lab
-        go = torch.ones(B, n_classes, N, device=vol.device)
-        gvol = torch.zeros(vol.shape, device=vol.device)
+        go = torch.ones(B, n_classes, N, device=vol.device, dtype=torch.float32)
+        gvol = torch.zeros(vol.shape, device=vol.device, dtype=torch.float32)
         timings = {}
         for mib in candidates:
             timings[mib] = self._time(

@@ -126,9 +126,9 @@ class BatchedRenderer:
             self.step.append(step)
         self.N = [r.height * r.width for r in requests]
         # static buffers
-        self.M = torch.zeros(R, 3, 4, device=self.device)
-        self.gM = torch.zeros(R, 3, 4, device=self.device)
-        self.gsrc = [torch.zeros(s.shape[1:], device=self.device) for s in self.src]
+        self.M = torch.zeros(R, 3, 4, device=self.device, dtype=torch.float32)
+        self.gM = torch.zeros(R, 3, 4, device=self.device, dtype=torch.float32)
+        self.gsrc = [torch.zeros(s.shape[1:], device=self.device, dtype=torch.float32) for s in self.src]
         self.offsets = np.concatenate([[0], np.cumsum([n * self.C for n in self.N])])
         self.out_flat = torch.empty(int(self.offsets[-1]), device=self.device, dtype=dt)
         self.go_flat = torch.zeros(int(self.offsets[-1]), device=self.device, dtype=dt)

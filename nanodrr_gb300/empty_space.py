@@ -126,13 +126,13 @@ class ProposalNetwork:
     def __init__(self, device, seed: int = 0):
         self.device = torch.device(device)
         g = torch.Generator().manual_seed(seed)
-        p = torch.zeros(PARAMS)
+        p = torch.zeros(PARAMS, dtype=torch.float32)
         # He-style init for the ReLU layers, small output layer
-        w1 = torch.randn(64, 64, generator=g) * math.sqrt(2.0 / 54)
+        w1 = torch.randn(64, 64, generator=g, dtype=torch.float32) * math.sqrt(2.0 / 54)
         w1[:, 54:] = 0.0
         p[0:4096] = w1.flatten()
-        p[4160:8256] = (torch.randn(64, 64, generator=g) * math.sqrt(2.0 / 64)).flatten()
-        p[8320:8448] = (torch.randn(2, 64, generator=g) * 0.01).flatten()
+        p[4160:8256] = (torch.randn(64, 64, generator=g, dtype=torch.float32) * math.sqrt(2.0 / 64)).flatten()
+        p[8320:8448] = (torch.randn(2, 64, generator=g, dtype=torch.float32) * 0.01).flatten()
         p[8448] = 0.0  # f_near bias: start wide (0 .. 1)
         p[8449] = 1.0
         self.params = p.to(self.device)
@@ -156,8 +156,8 @@ class ProposalNetwork:
         a.M, a.src, a.tgt = M.data_ptr(), src.data_ptr(), tgt.data_ptr()
         a.src_per_ray = 0 if src.shape[1] == 1 else 1
         a.B, a.N, a.width, a.n_samples = B, N, width, n_samples
-        X = torch.empty(B * N, FEATURES, device=vol.device)
-        T = torch.empty(B * N, 2, device=vol.device)
+        X = torch.empty(B * N, FEATURES, device=vol.device, dtype=torch.float32)
+        T = torch.empty(B * N, 2, device=vol.device, dtype=torch.float32)
         V = torch.empty(B * N, dtype=torch.uint8, device=vol.device)
         _prop_check(
             lib.ndrr_proposal_dataset(ctypes.byref(a), ctypes.c_void_p(extent.data_ptr()),
@@ -173,7 +173,7 @@ class ProposalNetwork:
         """One Adam step on a minibatch; returns the loss (device scalar)."""
         lib = _ffi.load()
         grads = torch.zeros_like(self.params)
-        loss = torch.zeros(1, device=self.device)
+        loss = torch.zeros(1, device=self.device, dtype=torch.float32)
         n = X.shape[0]
         count = max(1, n)
         st = ctypes.c_void_p(_stream(self.device))
@@ -201,7 +201,7 @@ class ProposalNetwork:
         """(grads [8450], loss) of the mean loss over the batch, no update."""
         lib = _ffi.load()
         grads = torch.zeros_like(self.params)
-        loss = torch.zeros(1, device=self.device)
+        loss = torch.zeros(1, device=self.device, dtype=torch.float32)
         n = X.shape[0]
         _prop_check(
             lib.ndrr_proposal_train_step(
@@ -216,7 +216,7 @@ class ProposalNetwork:
 
     def forward(self, X) -> torch.Tensor:
         """fp32 network outputs [R, 2] (the training-precision network)."""
-        out = torch.empty(X.shape[0], 2, device=self.device)
+        out = torch.empty(X.shape[0], 2, device=self.device, dtype=torch.float32)
         _prop_check(
             _ffi.load().ndrr_proposal_forward(
                 ctypes.c_void_p(self.params.data_ptr()), ctypes.c_void_p(X.data_ptr()), ctypes.c_int64(X.shape[0]),
@@ -245,7 +245,7 @@ class ProposalNetwork:
         for ep in range(epochs):
             perm = torch.randperm(n, device=self.device, generator=g)
             lr_ep = lr * (0.5 * (1 + math.cos(math.pi * ep / max(1, epochs))))  # cosine decay
-            tot = torch.zeros(1, device=self.device)
+            tot = torch.zeros(1, device=self.device, dtype=torch.float32)
             nb = 0
             for i in range(0, n, batch):
                 idx = perm[i : i + batch]
@@ -299,7 +299,7 @@ class EmptySpace:
 def extents(vol, M, src, tgt, step, n_samples, width) -> torch.Tensor:
     """Per-ray non-empty interval [B, N, 2] (in t) from the plain forward."""
     B, N, _ = tgt.shape
-    ext = torch.empty(B, N, 2, device=vol.device)
+    ext = torch.empty(B, N, 2, device=vol.device, dtype=torch.float32)
     raymarch_forward(vol, vol, M, src, tgt, step, n_samples, 1, width, extent=ext)
     return ext
 

@@ -78,7 +78,7 @@ def homography_resample_bwd(go: torch.Tensor, img: torch.Tensor, hom: torch.Tens
     go = go.float().contiguous()
     B, C, H, W = img.shape
     gimg = torch.zeros_like(img) if need_gimg else img.new_empty(0)
-    ghom = torch.empty(B, 3, 3, device=img.device) if need_ghom else img.new_empty(0)
+    ghom = torch.empty(B, 3, 3, device=img.device, dtype=torch.float32) if need_ghom else img.new_empty(0)
     lib = _ffi.load()
     nb = ctypes.c_uint64(0)
     _ffi.check(lib.ndrr_homography_resample_bwd_workspace_bytes(B, H, W, ctypes.byref(nb)), "workspace")
@@ -123,7 +123,7 @@ def _resample_op(img: torch.Tensor, k_old: torch.Tensor, k_new: torch.Tensor) ->
     img = img.contiguous()
     a, b = k_old.float().contiguous(), k_new.float().contiguous()
     B, C, H, W = img.shape
-    hom = torch.empty(B, 3, 3, device=img.device)
+    hom = torch.empty(B, 3, 3, device=img.device, dtype=torch.float32)
     out = torch.empty_like(img)
     _ffi.check(_ffi.load().ndrr_resample_fwd(img.data_ptr(), a.data_ptr(), a.shape[0], b.data_ptr(), b.shape[0], B, C,
                                              H, W, hom.data_ptr(), out.data_ptr(), _stream(img.device)),
@@ -143,7 +143,7 @@ def _resample_bwd(go: torch.Tensor, img: torch.Tensor, hom: torch.Tensor, k_old:
     a, b = k_old.float().contiguous(), k_new.float().contiguous()
     B, C, H, W = img.shape
     gimg = torch.zeros_like(img) if need_gimg else img.new_empty(0)
-    g_old, g_new = (torch.empty(B if need_gk else 0, 3, 3, device=img.device) for _ in range(2))
+    g_old, g_new = (torch.empty(B if need_gk else 0, 3, 3, device=img.device, dtype=torch.float32) for _ in range(2))
     lib = _ffi.load()
     nb = ctypes.c_uint64(0)
     _ffi.check(lib.ndrr_homography_resample_bwd_workspace_bytes(B, H, W, ctypes.byref(nb)), "workspace")
@@ -164,7 +164,7 @@ _resample_bwd_op = torch.library.custom_op("nanodrr_gb300::resample_bwd", mutate
 @_resample_bwd_op.register_fake
 def _(go, img, hom, k_old, k_new, need_gimg, need_gk):
     f = lambda t, on: t.new_empty(t.shape if on else (0,) + t.shape[1:], dtype=torch.float32)  # noqa: E731
-    gimg = torch.empty(img.shape, device=img.device) if need_gimg else img.new_empty(0)
+    gimg = torch.empty(img.shape, device=img.device, dtype=torch.float32) if need_gimg else img.new_empty(0)
     return gimg, f(k_old, need_gk), f(k_new, need_gk)
 
 

@@ -765,7 +765,7 @@ def _ex_bwd(
             "disable deterministic algorithms or detach the volume"
         )
     if need_gvol and not (need_gM or need_gcam) and n_classes == 1 and quad.numel():
-        none = [torch.empty(0, device=vol.device) for _ in range(4)]
+        none = [torch.empty(0, device=vol.device, dtype=torch.float32) for _ in range(4)]
         return volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo, slab_mib), *none
     if windows.numel():
         skip, win = None, windows
@@ -900,7 +900,7 @@ def _sums_bwd(go: torch.Tensor, vol: torch.Tensor, quad: torch.Tensor, M: torch.
     a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     _ffi.check(lib.ndrr_pose_from_sums(ctypes.byref(a), _ptr(sums), _stream_handle(dev)), "ndrr_pose_from_sums")
     if not need_gvol:
-        return torch.empty(0, device=dev), gM
+        return torch.empty(0, device=dev, dtype=torch.float32), gM
     return volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo, slab_mib), gM
 
 

@@ -91,7 +91,7 @@ def _pose_inputs(rot, xyz, rt_inv, pivot, pivot_inv):
 def _so3_pose_op(rot: torch.Tensor, xyz: torch.Tensor, rt_inv: torch.Tensor, pivot: torch.Tensor,
                  pivot_inv: torch.Tensor) -> torch.Tensor:
     B, rows, r, x, a, p, c = _pose_inputs(rot, xyz, rt_inv, pivot, pivot_inv)
-    pose = torch.empty(B, 4, 4, device=rt_inv.device)
+    pose = torch.empty(B, 4, 4, device=rt_inv.device, dtype=torch.float32)
     _ffi.check(_ffi.load().ndrr_pose_so3_fwd(r.data_ptr(), x.data_ptr(), rows, a.data_ptr(), p.data_ptr(),
                                              c.data_ptr(), B, pose.data_ptr(),
                                              _ffi.stream_handle(rt_inv.device)),
@@ -108,8 +108,8 @@ def _so3_pose_bwd(gpose: torch.Tensor, rot: torch.Tensor, xyz: torch.Tensor, rt_
                   pivot: torch.Tensor, pivot_inv: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     B, rows, r, x, a, p, c = _pose_inputs(rot, xyz, rt_inv, pivot, pivot_inv)
     g = gpose.float().contiguous()
-    g_rot = torch.empty(B, 3, device=rt_inv.device)
-    g_xyz = torch.empty(B, 3, device=rt_inv.device)
+    g_rot = torch.empty(B, 3, device=rt_inv.device, dtype=torch.float32)
+    g_xyz = torch.empty(B, 3, device=rt_inv.device, dtype=torch.float32)
     _ffi.check(_ffi.load().ndrr_pose_so3_bwd(g.data_ptr(), r.data_ptr(), x.data_ptr(), rows, a.data_ptr(),
                                              p.data_ptr(), c.data_ptr(), B, g_rot.data_ptr(), g_xyz.data_ptr(),
                                              _ffi.stream_handle(rt_inv.device)),
@@ -187,8 +187,8 @@ def _ncc_op(x1: torch.Tensor, x2: torch.Tensor, eps: float) -> tuple[torch.Tenso
     _ncc_check(x1, x2)
     B, C, H, W = x1.shape
     a, b = x1.float().contiguous(), x2.float().contiguous()
-    score = torch.empty(B, device=x1.device)
-    stats = torch.empty(B, C, 8, device=x1.device)
+    score = torch.empty(B, device=x1.device, dtype=torch.float32)
+    stats = torch.empty(B, C, 8, device=x1.device, dtype=torch.float32)
     lib = _ffi.load()
     nb = ctypes.c_uint64(0)
     _ffi.check(lib.ndrr_ncc_workspace_bytes(B, C, H * W, ctypes.byref(nb)), "ndrr_ncc_workspace_bytes")
@@ -276,7 +276,7 @@ def _ncc_patch_op(x1: torch.Tensor, x2: torch.Tensor, p: int, eps: float) -> tup
     """(score [B], window statistics [B, C, 5, H', W'] float64)."""
     B, C, H, W = x1.shape
     a, b = x1.float().contiguous(), x2.float().contiguous()
-    score = torch.empty(B, device=x1.device)
+    score = torch.empty(B, device=x1.device, dtype=torch.float32)
     maps = torch.empty(B, C, 5, H - p + 1, W - p + 1, device=x1.device, dtype=torch.float64)
     lib = _ffi.load()
     nb = ctypes.c_uint64(0)

@@ -159,9 +159,9 @@ def _ray_setup(k_inv, sdd, batch, height, width, n_samples, orthographic):
     """(src, tgt, step) of `batch` poses, expanded and contiguous."""
     k, s = k_inv.detach().contiguous(), sdd.detach().contiguous()
     N = height * width
-    tgt = torch.empty(batch, N, 3, device=k.device)
-    src = torch.empty(batch, N if orthographic else 1, 3, device=k.device)
-    step = torch.empty(batch, N, device=k.device)
+    tgt = torch.empty(batch, N, 3, device=k.device, dtype=torch.float32)
+    src = torch.empty(batch, N if orthographic else 1, 3, device=k.device, dtype=torch.float32)
+    step = torch.empty(batch, N, device=k.device, dtype=torch.float32)
     _ffi.check(
         _ffi.load().ndrr_ray_setup(k.data_ptr(), k.shape[0], s.data_ptr(), s.shape[0], batch, height, width,
                                    int(orthographic), n_samples, src.data_ptr(), tgt.data_ptr(), step.data_ptr(),
@@ -189,8 +189,8 @@ def _ray_setup_bwd(gsrc: torch.Tensor | None, gtgt: torch.Tensor | None, gstep: 
                    orthographic: bool) -> tuple[torch.Tensor, torch.Tensor]:
     k, s = k_inv.contiguous(), sdd.contiguous()
     grads = [None if g is None else g.float().contiguous() for g in (gsrc if orthographic else None, gtgt, gstep)]
-    g_k = torch.empty(batch, 3, 3, device=k.device)
-    g_s = torch.empty(batch, device=k.device)
+    g_k = torch.empty(batch, 3, 3, device=k.device, dtype=torch.float32)
+    g_s = torch.empty(batch, device=k.device, dtype=torch.float32)
     lib = _ffi.load()
     nb = ctypes.c_uint64(0)
     _ffi.check(lib.ndrr_ray_setup_bwd_workspace_bytes(batch, height, width, ctypes.byref(nb)), "workspace query")
@@ -245,8 +245,8 @@ def _affine_takes(w2v: torch.Tensor, rt_inv: torch.Tensor) -> bool:
 def _camera_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, low: bool) -> tuple[torch.Tensor, torch.Tensor]:
     w, rt = w2v.detach().contiguous(), rt_inv.detach().contiguous()
     B = rt.shape[0]
-    M = torch.empty(B, 3, 4, device=rt.device)
-    M_lo = torch.empty(B, 3, 4, device=rt.device) if low else M.new_empty(0)
+    M = torch.empty(B, 3, 4, device=rt.device, dtype=torch.float32)
+    M_lo = torch.empty_like(M) if low else M.new_empty(0)
     _ffi.check(_ffi.load().ndrr_camera_affine(w.data_ptr(), rt.data_ptr(), B, M.data_ptr(),
                                               M_lo.data_ptr() if low else None,
                                               _ffi.stream_handle(rt.device)), "ndrr_camera_affine")
@@ -266,7 +266,7 @@ def _(w2v, rt_inv):
 
 def _camera_affine_bwd(gM: torch.Tensor, w2v: torch.Tensor) -> torch.Tensor:
     g, w = gM.contiguous(), w2v.contiguous()
-    out = torch.empty(g.shape[0], 4, 4, device=g.device)
+    out = torch.empty(g.shape[0], 4, 4, device=g.device, dtype=torch.float32)
     _ffi.check(_ffi.load().ndrr_camera_affine_bwd(w.data_ptr(), g.data_ptr(), g.shape[0], out.data_ptr(),
                                                   _ffi.stream_handle(g.device)),
                "ndrr_camera_affine_bwd")
