@@ -1,4 +1,4 @@
-"""When an adjoint may be called without its operator.
+"""When a call may pass its operator by.
 
 The library's adjoints are registered operators, so that traced and transformed
 graphs see them; an operator call costs 100 to 150 us of host time on the Arm
@@ -14,15 +14,17 @@ _PLAIN = (torch.Tensor, torch.nn.Parameter)
 _dispatch_modes = getattr(torch._C, "_len_torch_dispatch_stack", None)
 _functorch = getattr(torch._C, "_functorch", None)
 _interpreters = getattr(_functorch, "peek_interpreter_stack", None)
+_legacy_batched = getattr(_functorch, "is_legacy_batchedtensor", None)
 
 
 def plain_eager(*tensors) -> bool:
-    """Ordinary tensors (no fake, functional or other subclass), no gradient
-    recorded (a double backward must meet the operator, which refuses it), no
-    compiler, dispatch mode or function transform active. Where this torch
-    cannot tell, the operator is called."""
-    if _dispatch_modes is None or _interpreters is None or torch.is_grad_enabled():
+    """Ordinary tensors (no fake, functional or other subclass, and not batched
+    by the vmap of torch.autograd.grad(is_grads_batched=True), which enters no
+    function transform), no gradient recorded (a double backward must meet the
+    operator, which refuses it), no compiler, dispatch mode or function
+    transform active. Where this torch cannot tell, the operator is called."""
+    if _dispatch_modes is None or _interpreters is None or _legacy_batched is None or torch.is_grad_enabled():
         return False
-    if any(t is not None and type(t) not in _PLAIN for t in tensors):
+    if any(t is not None and (type(t) not in _PLAIN or _legacy_batched(t)) for t in tensors):
         return False
     return not torch.compiler.is_compiling() and _dispatch_modes() == 0 and _interpreters() is None
