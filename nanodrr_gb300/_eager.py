@@ -17,14 +17,21 @@ _interpreters = getattr(_functorch, "peek_interpreter_stack", None)
 _legacy_batched = getattr(_functorch, "is_legacy_batchedtensor", None)
 
 
-def plain_eager(*tensors) -> bool:
+def plain_tensors(*tensors) -> bool:
     """Ordinary tensors (no fake, functional or other subclass, and not batched
     by the vmap of torch.autograd.grad(is_grads_batched=True), which enters no
-    function transform), no gradient recorded (a double backward must meet the
-    operator, which refuses it), no compiler, dispatch mode or function
-    transform active. Where this torch cannot tell, the operator is called."""
-    if _dispatch_modes is None or _interpreters is None or _legacy_batched is None or torch.is_grad_enabled():
+    function transform) with no compiler, dispatch mode or function transform
+    active: a launch may read their pointers. False where this torch cannot
+    tell."""
+    if _dispatch_modes is None or _interpreters is None or _legacy_batched is None:
         return False
     if any(t is not None and (type(t) not in _PLAIN or _legacy_batched(t)) for t in tensors):
         return False
     return not torch.compiler.is_compiling() and _dispatch_modes() == 0 and _interpreters() is None
+
+
+def plain_eager(*tensors) -> bool:
+    """Whether a backward may call the function behind its operator: plain
+    tensors and no gradient recorded (a double backward must meet the operator,
+    which refuses it)."""
+    return not torch.is_grad_enabled() and plain_tensors(*tensors)

@@ -19,7 +19,7 @@ import weakref
 import torch
 
 from . import _ffi
-from ._eager import plain_eager
+from ._eager import plain_eager, plain_tensors
 from .raymarch import (
     _SkipArgs,
     fused_raymarch_ex,
@@ -235,11 +235,11 @@ torch.library.register_autograd("nanodrr_gb300::ray_setup", _ray_setup_backward,
 # --------------------------------------------------------- camera -> voxel
 def _affine_takes(w2v: torch.Tensor, rt_inv: torch.Tensor) -> bool:
     """Float32 affine and poses on one CUDA device, the affine without a
-    gradient, outside tracing; others use `_affine_product`."""
-    return (not (hasattr(torch, "compiler") and torch.compiler.is_compiling())
-            and rt_inv.is_cuda and w2v.device == rt_inv.device and w2v.dtype == rt_inv.dtype == torch.float32
+    gradient, outside tracing and transforms (poses batched by vmap or fake
+    have no pointer to launch with); others use `_affine_product`."""
+    return (rt_inv.is_cuda and w2v.device == rt_inv.device and w2v.dtype == rt_inv.dtype == torch.float32
             and tuple(w2v.shape) == (4, 4) and rt_inv.dim() == 3 and rt_inv.shape[0] >= 1
-            and tuple(rt_inv.shape[1:]) == (4, 4) and not w2v.requires_grad)
+            and tuple(rt_inv.shape[1:]) == (4, 4) and not w2v.requires_grad and plain_tensors(w2v, rt_inv))
 
 
 def _camera_affine(w2v: torch.Tensor, rt_inv: torch.Tensor, low: bool) -> tuple[torch.Tensor, torch.Tensor]:
