@@ -23,11 +23,13 @@ def plain_tensors(*tensors) -> bool:
     function transform) with no compiler, dispatch mode or function transform
     active: a launch may read their pointers. False where this torch cannot
     tell."""
+    if torch.compiler.is_compiling():  # first: the compiler traces past it, not into the tests below
+        return False
     if _dispatch_modes is None or _interpreters is None or _legacy_batched is None:
         return False
     if any(t is not None and (type(t) not in _PLAIN or _legacy_batched(t)) for t in tensors):
         return False
-    return not torch.compiler.is_compiling() and _dispatch_modes() == 0 and _interpreters() is None
+    return _dispatch_modes() == 0 and _interpreters() is None
 
 
 def plain_eager(*tensors) -> bool:
