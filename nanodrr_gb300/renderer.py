@@ -354,11 +354,12 @@ def compact_label(subject: Subject) -> torch.Tensor:
     return packed
 
 
-def _batched(t: torch.Tensor, B: int) -> torch.Tensor:
-    """`t` expanded to B poses, float32 and contiguous (itself when it is)."""
-    if t.shape[0] == B and t.dtype == torch.float32 and t.is_contiguous():
+def _batched(t: torch.Tensor, B: int, dim: int) -> torch.Tensor:
+    """`t` expanded to B poses (a leading batch added where it has one dimension
+    less than `dim`), float32 and contiguous (itself when it is)."""
+    if t.dim() == dim and t.shape[0] == B and t.dtype == torch.float32 and t.is_contiguous():
         return t
-    return t.expand(B, *[-1] * (t.dim() - 1)).float().contiguous()
+    return t.expand(B, *[-1] * (dim - 1)).float().contiguous()
 
 
 def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) -> torch.Tensor:
@@ -401,9 +402,9 @@ def render_cuda(subject, rt_inv, src, tgt, step_size, n_samples, height, width) 
         vol,
         lab,
         M.contiguous(),
-        _batched(src, B),
-        _batched(tgt, B),
-        _batched(step_size, B),
+        _batched(src, B, 3),
+        _batched(tgt, B, 3),
+        _batched(step_size, B, 2),
         n_samples,
         C,
         width,
