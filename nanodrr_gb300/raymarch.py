@@ -541,7 +541,7 @@ def volume_gradient(go, vol, quad, M, src, tgt, step, n_samples, width, M_lo=Non
     a.go, a.go_dtype = _ptr(go), ndrr_dtype(go)
     a.need_gvol, a.gvol_overwrite = 1, 1
     a.gvol, a.gvol_quad, a.vol_quad = _ptr(gvol), gq.data_ptr(), quad.data_ptr()
-    quad_is_labeled(vol, quad)  # raises unless it is a quad copy of this volume
+    a.quad_labels = int(quad_is_labeled(vol, quad))  # refused: a labelled quad is for several classes
     # Without the volume's own lines in L2 beside them, slabs of 96 MiB of
     # gradient serve the scatter best (64 / 96 / 128 / 192 MiB: 4.51, 4.34, 4.44,
     # 4.67 ms at 512^3, 32 poses x 256^2 x 800; 0.383, 0.390, 0.404, 0.419 at
@@ -864,7 +864,7 @@ def fused_raymarch_sums(
     _set_M_lo(a, M_lo, M)
     a.out, a.out_dtype = _ptr(out), a.vol_dtype
     a.vol_quad = quad.data_ptr()
-    quad_is_labeled(vol, quad)
+    a.quad_labels = int(quad_is_labeled(vol, quad))  # refused: a labelled quad is for several classes
     skip = _skip_of(vol, occ_grid, occ_cell, proposal, skip_mode, margin)
     windows = skip_windows(vol, M, src, tgt, step, n_samples, width, skip) if skip is not None else None
     a.sample_window = _ptr(windows)
@@ -887,10 +887,18 @@ def _sums_bwd(go: torch.Tensor, vol: torch.Tensor, quad: torch.Tensor, M: torch.
             "Volume gradients on the cuda backend use nondeterministic atomics; "
             "disable deterministic algorithms or detach the volume"
         )
+    _check_inputs(vol, vol, M, src, tgt, step, n_samples, 1)
+    vol, _, M, src, tgt, step = _prep(vol, vol, M, src, tgt, step)
     go = go.contiguous() if go.dtype in _FLOAT_DTYPES else go.float().contiguous()
     B, N, _ = tgt.shape
+    if go.shape != (B, 1, N):
+        raise ValueError(f"go must be [B, 1, N] = [{B}, 1, {N}], got {tuple(go.shape)}")
+    if sums.shape != (6, B, N) or sums.dtype != torch.float32:
+        raise ValueError(f"sums must be float32 [6, B, N] = [6, {B}, {N}], got {sums.dtype} {tuple(sums.shape)}")
+    sums = sums.contiguous()
     dev = vol.device
-    gM = torch.empty(B, 3, 4, device=dev, dtype=torch.float32)
+    # no ray: nothing is launched, and the sum is zero
+    gM = (torch.empty if N else torch.zeros)(B, 3, 4, device=dev, dtype=torch.float32)
     a = _base_args(vol, vol, M, src, tgt, step, n_samples, 1, width)
     a.go, a.go_dtype, a.gM = _ptr(go), ndrr_dtype(go), _ptr(gM)
     lib = _ffi.load()
@@ -921,7 +929,9 @@ def _sums_setup_context(ctx, inputs, output):
     ctx.set_materialize_grads(False)
 
 
-def _sums_backward(ctx, go, _g_sums):
+def _sums_backward(ctx, go, g_sums):
+    if g_sums is not None:
+        raise RuntimeError("the sums of fused_raymarch_sums are for its own backward and have no gradient")
     if go is None:
         return (None,) * 15
     vol, quad, M, M_lo, src, tgt, step, sums = ctx.saved_tensors
