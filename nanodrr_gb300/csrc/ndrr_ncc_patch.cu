@@ -246,6 +246,15 @@ __global__ void __launch_bounds__(kPatchThreads) ncc_patch_bwd_kernel(const floa
 
 static size_t patch_smem(int p, int k) { return (size_t)k * (kPatchTY + p - 1) * kPatchTX * sizeof(double); }
 
+// Lets `kern` have the shared memory of the largest window (183 and 110 KB),
+// whatever this call's: the limit belongs to the device, and a call that set
+// its own would lower it between another host thread's setting and launch.
+template <typename K>
+static cudaError_t allow_largest(K kern, int k) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)patch_smem(NDRR_NCC_PATCH_MOST, k));
+}
+
 static int cover(int n, int t) { return (n + t - 1) / t; }
 
 static long long patch_tiles(int rows, int cols) {
@@ -261,7 +270,7 @@ cudaError_t launch_ncc_patch_fwd(const float* x1, const float* x2, int B, int C,
     const int HO = H - p + 1, WO = W - p + 1;
     const int tiles = (int)patch_tiles(HO, WO);
     const size_t smem = patch_smem(p, 5);
-    cudaError_t e = cudaFuncSetAttribute(ncc_patch_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_largest(ncc_patch_fwd_kernel, 5);
     if (e != cudaSuccess) return e;
     double* partials = reinterpret_cast<double*>(workspace);
     ncc_patch_fwd_kernel<<<(unsigned)((long long)B * C * tiles), kPatchThreads, smem, st>>>(
@@ -276,7 +285,7 @@ cudaError_t launch_ncc_patch_bwd(const float* go, const float* x1, const float* 
                                  int H, int W, int p, float* g1, float* g2, cudaStream_t st) {
     const int tiles = (int)patch_tiles(H, W);
     const size_t smem = patch_smem(p, 3);
-    cudaError_t e = cudaFuncSetAttribute(ncc_patch_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_largest(ncc_patch_bwd_kernel, 3);
     const double norm = (double)C * (H - p + 1) * (W - p + 1) * ((double)p * p);
     const unsigned grid = (unsigned)((long long)B * C * tiles);
     for (int which = 0; which < 2 && e == cudaSuccess; ++which) {
