@@ -5,16 +5,22 @@
 // the score of a batch element is the mean over its planes' pixels of the
 // product.
 //
-// Forward: chunks of 1024 pixels per CTA accumulate the raw moments in pairs
-// of floats (error-free products and sums, about 48 bits, so centring after
-// the fact keeps full fp32 accuracy), a warp per plane sums the chunks in a
+// Forward: chunks of 1024 pixels per CTA accumulate moments about the chunk's
+// first pixel in pairs of floats (Knuth's error-free sum and difference, and
+// products by a fused multiply-add; about 46 bits) and shift them to raw
+// moments in fp64, so centring after the fact is as accurate as with moments
+// summed in fp64: the pairs' error is relative to the chunk's own spread about
+// one of its pixels, not to its offset. A warp per plane sums the chunks in a
 // fixed order in fp64 and forms the centred statistics (and, with one plane
 // per batch element, the score), and a CTA per batch element sums several
 // planes. The adjoint is the closed form of d score / d x, elementwise from
 // the saved statistics.
 //
 // The pairs are there because the fp64 pipe (2 lanes per clock and SM) bound
-// the moments: 8 x 1024^2 took 139 us in fp64, 39 us so (10 at memory speed).
+// the moments: 8 x 1024^2 took 139 us in fp64, 45 so (10 at memory speed).
+// Raw moments in pairs (36 us) lost a tenth of fp64's accuracy where the mean is
+// large: error of the score 8e-8, 8e-6 at means of 1e4, 1e5 standard
+// deviations, in fp64 and about the first pixel 1e-8, 6e-7.
 #include <cuda_runtime.h>
 
 #include "../../include/nanodrr_gb300.h"
@@ -30,19 +36,30 @@ constexpr int kNccBwdChunk = 4096;   // pixels per CTA of the adjoint
 static int ncc_chunks(int N) { return (N + kNccChunk - 1) / kNccChunk; }
 static int ncc_bwd_chunks(int N) { return (N + kNccBwdChunk - 1) / kNccBwdChunk; }
 
+// x + err without rounding (up to the pair's 46 bits): a float and what it lacks.
+struct Pair {
+    float x, err;
+};
+
+__device__ __forceinline__ Pair pair_diff(float a, float b) {  // a - b
+    const float d = __fsub_rn(a, b), bb = __fsub_rn(d, a);
+    return {d, __fsub_rn(__fsub_rn(a, __fsub_rn(d, bb)), __fadd_rn(b, bb))};
+}
+
+__device__ __forceinline__ Pair pair_product(Pair a, Pair b) {
+    const float p = __fmul_rn(a.x, b.x);
+    return {p, __fmaf_rn(a.x, b.err, __fmaf_rn(a.err, b.x, __fmaf_rn(a.x, b.x, -p)))};
+}
+
 // Sum kept as hi + lo: each term's rounding error against hi goes into lo.
 struct PairSum {
     float hi, lo;
-    __device__ __forceinline__ void add(float x, float err) {
-        const float s = __fadd_rn(hi, x);
+    __device__ __forceinline__ void add(Pair t) {
+        const float s = __fadd_rn(hi, t.x);
         const float bb = __fsub_rn(s, hi);
-        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(x, bb));
+        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(t.x, bb));
         hi = s;
-        lo = __fadd_rn(lo, __fadd_rn(e, err));
-    }
-    __device__ __forceinline__ void add_product(float x, float y) {
-        const float p = __fmul_rn(x, y);
-        add(p, __fmaf_rn(x, y, -p));
+        lo = __fadd_rn(lo, __fadd_rn(e, t.err));
     }
 };
 
@@ -60,6 +77,7 @@ __global__ void __launch_bounds__(kNccMomentBlock) ncc_moments_kernel(const floa
     const int beg = chunk * kNccChunk, end = min(N, beg + kNccChunk);
     const float* a = x1 + plane * N;
     const float* b = x2 + plane * N;
+    const float c1 = __ldg(a + beg), c2 = __ldg(b + beg);
     PairSum s[5] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
     bool plain = true;
 #pragma unroll 4
@@ -67,11 +85,12 @@ __global__ void __launch_bounds__(kNccMomentBlock) ncc_moments_kernel(const floa
         const float u = __ldg(a + i), v = __ldg(b + i);
         plain &= (u == 0.f || (fabsf(u) > 1e-15f && fabsf(u) < 1e16f)) &&
                  (v == 0.f || (fabsf(v) > 1e-15f && fabsf(v) < 1e16f));
-        s[0].add(u, 0.f);
-        s[1].add(v, 0.f);
-        s[2].add_product(u, u);
-        s[3].add_product(v, v);
-        s[4].add_product(u, v);
+        const Pair d = pair_diff(u, c1), e = pair_diff(v, c2);
+        s[0].add(d);
+        s[1].add(e);
+        s[2].add(pair_product(d, d));
+        s[3].add(pair_product(e, e));
+        s[4].add(pair_product(d, e));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool all_plain = __syncthreads_and(plain) != 0;
@@ -83,7 +102,7 @@ __global__ void __launch_bounds__(kNccMomentBlock) ncc_moments_kernel(const floa
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const float h = __shfl_xor_sync(0xffffffffu, t.hi, o), l = __shfl_xor_sync(0xffffffffu, t.lo, o);
-                t.add(h, l);
+                t.add({h, l});
             }
             x = (double)t.hi + (double)t.lo;
         } else {
@@ -98,9 +117,22 @@ __global__ void __launch_bounds__(kNccMomentBlock) ncc_moments_kernel(const floa
     }
     __syncthreads();
     if (threadIdx.x < 5) {
-        double x = 0.0;
-        for (int w = 0; w < kNccMomentBlock / 32; ++w) x += sh[w][threadIdx.x];
-        partials[(plane * nch + chunk) * 5 + threadIdx.x] = x;
+        const int k = threadIdx.x;
+        const int l = k == 3 ? 1 : k == 4 ? 1 : 0, r = k == 3 ? 1 : 0;  // first moments of a product's factors
+        double x = 0.0, sl = 0.0, sr = 0.0;
+        for (int w = 0; w < kNccMomentBlock / 32; ++w) {
+            x += sh[w][k];
+            sl += sh[w][l];
+            sr += sh[w][r];
+        }
+        if (all_plain) {  // sum (c + d) = sum d + n c; sum (c + d)(f + e) = sum d e + f sum d + c (sum e + n f)
+            const double n = (double)(end - beg), cl = (double)(l ? c2 : c1), cr = (double)(r ? c2 : c1);
+            if (k < 2)
+                x += n * (double)(k ? c2 : c1);
+            else
+                x += cl * sr + cr * (sl + n * cl);
+        }
+        partials[(plane * nch + chunk) * 5 + k] = x;
     }
 }
 
