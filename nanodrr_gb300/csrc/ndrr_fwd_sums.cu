@@ -144,8 +144,12 @@ __global__ void __launch_bounds__(256) pose_sums_kernel(const MarchParams p, con
 
 template <typename VT>
 static cudaError_t fwd_sums(const MarchParams& p, float* sums, cudaStream_t st) {
+    const KernelEvents& ev = kernel_events();
+    if (ev.start != nullptr) cudaEventRecord(ev.start, st);
     raymarch_fwd_sums_kernel<VT><<<(unsigned)((size_t)p.B * p.tm.tiles), (unsigned)(p.tw * p.th), 0, st>>>(p, sums);
-    return cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (ev.stop != nullptr && e == cudaSuccess) e = cudaEventRecord(ev.stop, st);
+    return e;
 }
 
 cudaError_t launch_fwd_sums(const ndrr_raymarch_args& a, LaunchShape ls, float* sums, cudaStream_t st) {

@@ -527,8 +527,12 @@ cudaError_t launch_scatter_slab(const ndrr_raymarch_args& a, const LaunchShape& 
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)std::max(1, sms * std::max(per_sm, 1));
+    const KernelEvents& ev = kernel_events();
+    if (ev.start != nullptr) cudaEventRecord(ev.start, st);
     kern<<<grid, block, 0, st>>>(p, s);
-    return cudaGetLastError();
+    e = cudaGetLastError();
+    if (ev.stop != nullptr && e == cudaSuccess) e = cudaEventRecord(ev.stop, st);
+    return e;
 }
 
 // Slab-ordered adjoint with volume gradient for the quad layout; writes gM
