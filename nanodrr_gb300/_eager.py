@@ -12,24 +12,30 @@ import torch
 
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 _dispatch_modes = getattr(torch._C, "_len_torch_dispatch_stack", None)
-_functorch = getattr(torch._C, "_functorch", None)
-_interpreters = getattr(_functorch, "peek_interpreter_stack", None)
-_legacy_batched = getattr(_functorch, "is_legacy_batchedtensor", None)
+_interpreters = getattr(getattr(torch._C, "_functorch", None), "peek_interpreter_stack", None)
+_key_included = getattr(torch._C, "_dispatch_tls_is_dispatch_key_included", None)
+try:
+    # Set while torch.autograd.grad(is_grads_batched=True) batches, which enters
+    # no function transform. One question per call: asking each tensor whether
+    # it is batched (is_legacy_batchedtensor) took 5 % of a small step.
+    _LEGACY_VMAP = torch._C._parse_dispatch_key("VmapMode")
+    _key_included(_LEGACY_VMAP)
+except Exception:  # not in this torch
+    _LEGACY_VMAP = None
 
 
 def plain_tensors(*tensors) -> bool:
-    """Ordinary tensors (no fake, functional or other subclass, and not batched
-    by the vmap of torch.autograd.grad(is_grads_batched=True), which enters no
-    function transform) with no compiler, dispatch mode or function transform
-    active: a launch may read their pointers. False where this torch cannot
-    tell."""
+    """Ordinary tensors (no fake, functional or other subclass) with no
+    compiler, dispatch mode, function transform or batching active: a launch may
+    read their pointers. False where this torch cannot tell."""
     if torch.compiler.is_compiling():  # first: the compiler traces past it, not into the tests below
         return False
-    if _dispatch_modes is None or _interpreters is None or _legacy_batched is None:
+    if _dispatch_modes is None or _interpreters is None or _LEGACY_VMAP is None:
         return False
-    if any(t is not None and (type(t) not in _PLAIN or _legacy_batched(t)) for t in tensors):
-        return False
-    return _dispatch_modes() == 0 and _interpreters() is None
+    for t in tensors:
+        if type(t) not in _PLAIN and t is not None:
+            return False
+    return _dispatch_modes() == 0 and _interpreters() is None and not _key_included(_LEGACY_VMAP)
 
 
 def plain_eager(*tensors) -> bool:
