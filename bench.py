@@ -41,12 +41,12 @@ import torch  # noqa: E402
 
 BASELINE_HEADLINE = None  # no published number exists for this metric
 METRIC = "fwd+bwd DRR frames/s at 512^3/256^2, learned-skip vs plain kernel"
-# DRAM read + write bytes per sample of the slab-ordered adjoint kernel,
+# DRAM read + write bytes per sample of the two volume-gradient kernels,
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of one launch)
-# on a 384^3 x 8-pose case of the same kernel and scaled here by the samples
-# of a launch.
-SLAB_DRAM_BYTES_PER_SAMPLE = 19.67
-SLAB_DRAM_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch, 384^3 x 8 poses, scaled per sample"
+# on 384^3 cases of the same kernels and scaled here by the samples of a launch.
+SCATTER_DRAM_BYTES_PER_SAMPLE = 9.13  # 16 poses, columns of four rays per thread
+SLAB_DRAM_BYTES_PER_SAMPLE = 19.67  # 8 poses
+DRAM_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch, 384^3, scaled per sample"
 
 
 def parse_args():
@@ -264,9 +264,15 @@ def run_ours(args, world, rank, local):
     import nanodrr_gb300 as nd
     from nanodrr_gb300 import _build
     from nanodrr_gb300.empty_space import EmptySpace, train_proposal
-    from nanodrr_gb300.raymarch import raymarch_backward, raymarch_forward, skip_windows
+    from nanodrr_gb300.raymarch import (
+        fused_raymarch_sums,
+        raymarch_backward,
+        raymarch_forward,
+        skip_windows,
+        volume_gradient,
+    )
     from nanodrr_gb300.registration import GraphedStep, NormalizedCrossCorrelation2d, Registration
-    from nanodrr_gb300.renderer import _affine_product, _make_src, _make_tgt, cached_quad
+    from nanodrr_gb300.renderer import _SUMS_RAYS, _affine_product, _make_src, _make_tgt, cached_quad
 
     _build.build()
     dev = torch.device("cuda", local)
@@ -423,6 +429,13 @@ def run_ours(args, world, rank, local):
                                       quad=quad), reps)
         fwd_kernel_ms = _kernel_only_ms(lambda: raymarch_forward(vol, vol, M, srcb, tgtb, stepsz, S, 1, Hd,
                                                                  quad=quad), reps)
+        # what the step runs from renderer._SUMS_RAYS rays on: the forward that
+        # leaves the pose sums, and the volume gradient's scatter by itself
+        e8 = torch.empty(0, dtype=torch.uint8, device=dev)
+        sums_kernel_ms = _kernel_only_ms(
+            lambda: fused_raymarch_sums(vol, quad, M, e8.float(), srcb, tgtb, stepsz, S, Hd, e8, 0, e8, 0, 0.0, 0), reps)
+        scatter_kernel_ms = _kernel_only_ms(lambda: volume_gradient(go, vol, quad, M, srcb, tgtb, stepsz, S, Hd), reps)
+        scatter_call_ms = _event_ms(lambda: volume_gradient(go, vol, quad, M, srcb, tgtb, stepsz, S, Hd), reps)
         l2 = l2_read_peak(dev)
         red = reduction_peak(dev)
         times = {"fwd": [], "fwd_learned": [], "bwd": [], "fwd_plain_layout": [], "bwd_plain_layout": [],
@@ -457,20 +470,25 @@ def run_ours(args, world, rank, local):
                 times["bwd_direct"].append(e[6].elapsed_time(e[7]))
     e_bytes = vol.element_size()
     fwd_bytes = n_samp * 8 * e_bytes
-    bwd_bytes = n_samp * (8 * e_bytes + 4 + 8 * 4 * 2)
+    scatters = B * Hd * Hd >= _SUMS_RAYS
+    # the scatter reads no corners and the upstream gradient once a ray
+    bwd_bytes = n_samp * 8 * 4 * 2 + (4 * B * Hd * Hd if scatters else n_samp * (8 * e_bytes + 4))
     fwd_s = statistics.median(times["fwd"]) / 1e3
     bwd_s = statistics.median(times["bwd"]) / 1e3
     fwdl_s = statistics.median(times["fwd_learned"]) / 1e3
-    kern_s = bwd_kernel_ms / 1e3
+    main_ms = scatter_kernel_ms if scatters else bwd_kernel_ms
+    kern_s = main_ms / 1e3
     peaks = _peaks()
-    traffic = SLAB_DRAM_BYTES_PER_SAMPLE * n_samp
+    traffic = (SCATTER_DRAM_BYTES_PER_SAMPLE if scatters else SLAB_DRAM_BYTES_PER_SAMPLE) * n_samp
     dram_gbs = traffic / kern_s / 1e9
     demand_gbs = bwd_bytes / kern_s / 1e9
     st = stats.tolist()
     ost = occ_stats.tolist()
     roofline = {
         "bound": "hbm",
-        "kernel": "raymarch_bwd_slab_kernel (adjoint with pose and volume gradient, slab-ordered, quad layout)",
+        "kernel": ("raymarch_scatter_slab_kernel (volume gradient from sample positions, slab-ordered, quad layout)"
+                   if scatters else
+                   "raymarch_bwd_slab_kernel (adjoint with pose and volume gradient, slab-ordered, quad layout)"),
         "timed": "the march kernel alone (CUDA events the library records around it on the launch stream)",
         # DRAM bytes of one launch per kernel time, against the measured HBM
         # copy bandwidth: the fraction of HBM the kernel uses
@@ -480,27 +498,32 @@ def run_ours(args, world, rank, local):
         "unit": "GB/s",
         "frac": round(dram_gbs / peaks["hbm_gbs"], 4),
         "traffic": round(traffic, 1),
-        "traffic_source": SLAB_DRAM_SOURCE,
-        # the per-sample demand bytes (8 corner reads, the upstream gradient,
-        # 8 corner read-modify-writes), mostly served by L1 and L2, against the
-        # L2 read bandwidth measured by the library's probe in this run
+        "traffic_source": DRAM_SOURCE,
+        # the demand bytes (8 corner read-modify-writes a sample; for the slab
+        # adjoint also 8 corner reads and the upstream gradient), mostly served
+        # by L1 and L2, against the L2 read bandwidth measured by the library's
+        # probe in this run
         "algorithmic_bytes_per_launch": bwd_bytes,
         "demand_gbs": round(demand_gbs, 1),
         "l2_peak_gbs": l2["gbs"],
         "l2_peak_how": l2["how"],
         "l2_frac": round(demand_gbs / l2["gbs"], 4) if l2["gbs"] else None,
         "samples_per_launch": n_samp,
-        "kernel_ms": round(bwd_kernel_ms, 3),
-        "call_ms": round(bwd_s * 1e3, 3),
+        "kernel_ms": round(main_ms, 3),
+        "call_ms": round(scatter_call_ms if scatters else bwd_s * 1e3, 3),
+        "fwd_sums_kernel_ms": round(sums_kernel_ms, 3),
+        "slab_adjoint_kernel_ms": round(bwd_kernel_ms, 3),
+        "slab_adjoint_call_ms": round(bwd_s * 1e3, 3),
         "fwd_kernel_ms": round(fwd_kernel_ms, 3),
         "fwd_ms": round(fwd_s * 1e3, 3),
         "fwd_learned_ms": round(fwdl_s * 1e3, 3),
         "learned_windows_ms": round(statistics.median(times["learned_windows"]), 3),
         "fwd_gsamples_per_s": round(n_samp / fwd_s / 1e9, 2),
         "bwd_gsamples_per_s": round(n_samp / kern_s / 1e9, 2),
-        # the scatter's two 16-byte reductions per sample alone, into an
-        # L2-resident array (library probe, this run): the ceiling the
-        # adjoint's sample rate is bound by
+        # two 16-byte reductions per sample alone, into an L2-resident array
+        # (library probe, this run). The scatter merges the terms of
+        # neighbouring rays before it reduces them, so the probe's rate of
+        # samples is not its ceiling.
         "reduction_peak_gsamples_per_s": red["gsamples_per_s"],
         "reduction_peak_how": red["how"],
         "reduction_frac": round(n_samp / kern_s / 1e9 / red["gsamples_per_s"], 4) if red["gsamples_per_s"] else None,
@@ -614,11 +637,13 @@ def run_ours(args, world, rank, local):
         "roofline": roofline,
         "adjoint_warp_aggregation": warp_agg,
         "e2e": e2e,
-        # per step: pose, [proposal network and window check (learned)],
-        # forward march, NCC moments, statistics, score and adjoint, slab
-        # plan, scan and fill, adjoint march, per-pose reduction,
-        # quad-gradient fold, pose adjoint
-        "gpu_launches": (15 if headline == "learned" else 13) * args.steps,
+        # per step: pose, ray set-up (graphed; an eager step takes cached rays),
+        # camera affine, [sample windows, proposal network], forward march, NCC
+        # moments, statistics and adjoint, slab plan, scan and fill, volume
+        # march, fold, two pose reductions (the slab adjoint has one, and reads
+        # no pose sums), affine and pose adjoints
+        "gpu_launches": ((16 if scatters else 14) - (1 if args.no_graph else 0)
+                         + {"plain": 0, "occupancy": 1, "learned": 2}[headline]) * args.steps,
         "clocks": clk,
     }
     if cpu is not None:
