@@ -5,10 +5,12 @@
 // them: the adjoint then reads 24 bytes per ray instead of marching the
 // volume a second time (pose_sums_kernel). Positions, cells and gradients are
 // those of the adjoint (32.32 fixed point, ndrr_march.cuh). The image takes the
-// same corners at the forward's float positions, so that it is the image of a
-// render without a gradient (the two positions differ by an ulp of the float;
-// where that puts them on two sides of a cell face, the image extrapolates this
-// cell by as much).
+// same corners at the forward's float positions. It is not bitwise the image of
+// a render without a gradient: the two positions differ by an ulp of the float,
+// and where that puts them on two sides of a cell face, this image extrapolates
+// its cell by as much, while the plain one is in the next cell. The two are
+// equally far from the exact image and up to 2e-6 of the maximum apart on smooth
+// volumes, 4e-6 on white noise.
 //
 // Both marches wait for the same gathers, so the one that does both costs about
 // what the adjoint alone does (kernels alone): 16 poses x 200^2 x 500 samples of
@@ -20,7 +22,11 @@ namespace ndrr {
 
 // The trilinear derivative (cell_grad) from first differences of the corners
 // and their differences, which the three components share: 20 operations where
-// each component interpolated by itself takes 33.
+// each component interpolated by itself takes 33 (with those the kernel's steps
+// take 1.18 times as long at 8 x 1024^2 x 1000, 1.06 at 32 x 256^2 x 800 of
+// 512^3). dL/dM is as accurate with either, and as the marching adjoint's: root
+// mean square error against float64 over 12 seeded volumes and poses at four
+// sizes 1.38e-7 (16 x 181^2: 1.05e-7) for 1.26e-7 (1.14e-7).
 __device__ __forceinline__ void cell_grad_shared(const Cell& c, float& gx, float& gy, float& gz) {
     const float x00 = c.v001 - c.v000, x01 = c.v011 - c.v010;  // d/dx at (z, y) = (0, 0), (0, 1)
     const float x10 = c.v101 - c.v100, x11 = c.v111 - c.v110;

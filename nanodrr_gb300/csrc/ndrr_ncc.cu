@@ -18,9 +18,9 @@
 //
 // The pairs are there because the fp64 pipe (2 lanes per clock and SM) bound
 // the moments: 8 x 1024^2 took 139 us in fp64, 45 so (10 at memory speed).
-// Raw moments in pairs (36 us) lost a tenth of fp64's accuracy where the mean is
-// large: error of the score 8e-8, 8e-6 at means of 1e4, 1e5 standard
-// deviations, in fp64 and about the first pixel 1e-8, 6e-7.
+// Raw moments in pairs (36 us) are a tenth as accurate where the mean is large:
+// error of the score 8e-8, 8e-6 at means of 1e4, 1e5 standard deviations, in
+// fp64 and about the first pixel 1e-8, 6e-7.
 #include <cuda_runtime.h>
 
 #include "../../include/nanodrr_gb300.h"

@@ -515,7 +515,18 @@ cudaError_t launch_scatter_slab(const ndrr_raymarch_args& a, const LaunchShape& 
     const int R = p.tw * p.th;
     // Rays per thread: columns of four where the launch has rays enough to fill
     // the GPU four times over with them (about 2^18 resident rays at 12 warps per
-    // SM), else of two, where the tile splits into whole warps of them.
+    // SM), else of two, where the tile splits into whole warps of them. Kernel
+    // alone, ms with two / four (poses x detector, 500 samples):
+    //                    128^3          277 x 250 x 301   512^3
+    //    4 x 256^2      0.250 / 0.184   0.315 / 0.322   0.741 / 0.815
+    //    9 x 200^2      0.289 / 0.311   0.412 / 0.420   0.983 / 1.135
+    //    8 x 256^2      0.385 / 0.328   0.510 / 0.475   0.981 / 1.012
+    //   16 x 256^2      0.729 / 0.606   0.965 / 0.844   1.513 / 1.509  (2^20)
+    //   20 x 256^2      0.870 / 0.725   1.186 / 1.020   1.829 / 1.812
+    //    1 x 1024^2     0.758 / 0.455   0.881 / 0.684   1.270 / 1.675
+    //    4 x 1024^2     2.749 / 1.759   3.508 / 2.720   4.961 / 6.199
+    // From 2^20 rays four are ahead but for dense detectors over a large volume
+    // (last column), where two would be; below, the two sides cross by size.
     const long long rays = (long long)a.B * a.N;
     const int nc = rays >= (1 << 20) && R % 128 == 0 ? 4 : R % 64 == 0 ? 2 : 1;
     auto kern = nc == 4 ? raymarch_scatter_slab_kernel<4>

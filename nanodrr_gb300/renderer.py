@@ -40,13 +40,24 @@ _BACKENDS = ("auto", "cuda", "triton")
 _RAY_CACHE: dict = {}
 _RAY_CACHE_SIZE = 4
 
-# Rays from which a one-channel render that needs a pose gradient takes the
-# forward that leaves the pose sums (`fused_raymarch_sums`). Above it the
-# second march it saves is half of the step (16 poses x 200^2 x 500 samples:
-# 1.42 -> 0.76 ms of kernels, the step 1.48 -> 1.10 ms). Below, both marches
-# together are some tenths of a millisecond in a step that its host time bounds,
-# and the sums of few rays in another order would move the ill-conditioned
-# rotation gradient of a single pose at the 1e-5 level.
+# Rays (of all poses together) from which a one-channel render that needs a
+# pose gradient takes the forward that leaves the pose sums
+# (`fused_raymarch_sums`). Kernels of a pose step, with sums / with two marches,
+# us, and of its forward alone (500 samples of 512 x 512 x 400, float32):
+#   1 x 200^2   143 /  190   forward 126 /   95
+#   4 x 128^2   174 /  419           158 /  203
+#   8 x 200^2   399 /  690           380 /  321
+#  32 x 120^2  1506 / 3018          1491 / 1536
+#  16 x 200^2   768 / 1493           751 /  741
+#   4 x 512^2   802 / 1306           781 /  528
+# (250 of 128^3: 1 x 200^2 30 / 32 and 18 / 16, 16 x 200^2 79 / 104 and 63 / 46.)
+# The step gains at every size measured, so the line is not where the sums start
+# to pay. It keeps them out of small renders, where sums in another order would
+# move the ill-conditioned rotation gradient of a single pose at the 1e-5 level,
+# and where the gain is little of a step of 0.6 ms or more of host time; a batch
+# of small renders below it (32 x 120^2) would gain too. A forward whose
+# backward never runs pays for the sums, up to 1.6 times: evaluations of the loss
+# alone belong under torch.no_grad.
 _SUMS_RAYS = 1 << 19
 
 # Camera -> voxel affines of recent calls without a gradient, keyed by the
