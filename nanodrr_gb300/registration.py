@@ -260,6 +260,7 @@ def _patch_kernel_takes(x1: torch.Tensor, x2: torch.Tensor, p) -> bool:
     empty batches, other types, and the inputs that raise) is unfolded."""
     return (
         isinstance(p, int)
+        and not isinstance(p, bool)  # refused by unfold
         and x1.is_cuda
         and x1.device == x2.device
         and x1.dim() == 4

@@ -4,7 +4,7 @@ around them, against the unfolded windows."""
 import pytest
 import torch
 
-from nanodrr_gb300.registration import _to_patches, ncc_patch_score, ncc_score
+from nanodrr_gb300.registration import NormalizedCrossCorrelation2d, _to_patches, ncc_patch_score, ncc_score
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +53,9 @@ def test_windows_of_one_value():
     assert float((s.detach().cpu().double() - r.detach()).abs().max()) <= 1e-5
     for u, v in ((a.grad, c.grad), (b.grad, d.grad)):
         assert float((u.cpu().double() - v).abs().max()) <= 1e-5 * float(v.abs().max())
+
+
+def test_a_window_size_of_true_is_refused():
+    x = torch.rand(1, 1, 8, 8, device="cuda")
+    with pytest.raises(TypeError):
+        NormalizedCrossCorrelation2d(patch_size=True)(x, x)
